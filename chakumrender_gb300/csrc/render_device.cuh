@@ -194,6 +194,7 @@ struct LightQuery {
   float d;
   F3 Le;
   bool hit;
+  uint32_t mesh;  // the triangle met of the first MESH light (in list order) that is met; kMiss: none
 };
 
 // Light kinds a shading kernel is compiled for: kernels for scenes whose lights
@@ -211,6 +212,7 @@ __device__ __forceinline__ LightQuery query_lights(const ShadeView &sv, F3 x, F3
   q.d = 3.0e38f;
   q.Le = f3(0.f, 0.f, 0.f);
   q.hit = false;
+  q.mesh = kMiss;
   RayPre r = ray_pre(o_off, w, 0.f);
   for (uint32_t k = 0; k < sv.nlights; ++k) {
     DevLight L = sv.lights[k];
@@ -218,6 +220,7 @@ __device__ __forceinline__ LightQuery query_lights(const ShadeView &sv, F3 x, F3
       float t;
       uint32_t id = light_tri_hit(sv, L, r, t);
       if (id == kMiss) continue;
+      if (q.mesh == kMiss && L.type == CKR_LIGHT_MESH) q.mesh = id;
       F3 ne = tri_normal(sv, id);
       float c1 = fabsf(dot(w, ne));
       q.pdf_sum += (float)n_per_light * (t * t) / (c1 * L.area);

@@ -18,8 +18,8 @@ struct DevLight {
   uint32_t count;    // MESH: emitter triangles
   uint32_t cdf;      // MESH: offset of its 300-entry inverse CDF in the cdf table
   float area;        // MESH/TRI: total emitter area (the pdf's 1/area)
-  float px, py, pz;  // POINT: position; SPHERE: centre
-  float radius;      // SPHERE
+  float px, py, pz;  // POINT: position; SPHERE: centre; MESH/TRI: centre of a sphere around its triangles
+  float radius;      // SPHERE; MESH/TRI: radius of that sphere
   float pr, pg, pb;  // POINT: power
   uint32_t pcdf;     // MESH/TRI: offset of its per-triangle power CDF (one-sample NEE)
   float power;       // MESH/TRI: emitted power sum of luminance(radiance) x area

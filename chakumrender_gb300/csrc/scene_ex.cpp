@@ -133,6 +133,28 @@ int build_env(const ckr_env_light &e, EnvTables &t) {
   return CKR_OK;
 }
 
+// A sphere around the triangles [first, first + count) (MESH/TRI lights): the centre of
+// their box, the largest distance of a corner from it, rounded up.
+void bounding_sphere(const float *tri9, uint32_t first, uint32_t count, DevLight &g) {
+  const float *v = tri9 + 9 * (size_t)first;
+  const size_t n = 3 * (size_t)count;
+  float lo[3] = {v[0], v[1], v[2]}, hi[3] = {v[0], v[1], v[2]};
+  for (size_t i = 0; i < n; ++i)
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = std::min(lo[c], v[3 * i + c]);
+      hi[c] = std::max(hi[c], v[3 * i + c]);
+    }
+  g.px = 0.5f * (lo[0] + hi[0]);
+  g.py = 0.5f * (lo[1] + hi[1]);
+  g.pz = 0.5f * (lo[2] + hi[2]);
+  double r2 = 0;
+  for (size_t i = 0; i < n; ++i) {
+    const double x = (double)v[3 * i] - g.px, y = (double)v[3 * i + 1] - g.py, z = (double)v[3 * i + 2] - g.pz;
+    r2 = std::max(r2, x * x + y * y + z * z);
+  }
+  g.radius = (float)(std::sqrt(r2) * (1.0 + 1e-6));
+}
+
 template <typename T>
 int upload(DevBuf<T> &buf, const T *src, size_t n) {
   if (buf.reserve(n ? n : 1) != cudaSuccess) return CKR_ERR_OUT_OF_MEMORY;
@@ -172,10 +194,12 @@ extern "C" int ckr_scene_create_ex(const ckr_scene_desc *d, ckr_scene **out) {
       g.cdf = (uint32_t)cdf.size();
       cdf.resize(cdf.size() + kInvCdfBins);
       g.area = (float)build_inv_cdf(d->tri9, L.first, L.count, &cdf[g.cdf]);
+      bounding_sphere(d->tri9, L.first, L.count, g);
     } else if (L.type == CKR_LIGHT_TRI) {
       if (L.first >= d->ntri) return CKR_ERR_INVALID_ARGUMENT;
       g.count = 1;
       g.area = (float)tri_area(d->tri9 + 9 * (size_t)L.first);
+      bounding_sphere(d->tri9, L.first, 1, g);
     } else if (L.type == CKR_LIGHT_SPHERE) {
       if (L.first >= d->nsph) return CKR_ERR_INVALID_ARGUMENT;
       const float *s = d->sph4 + 4 * (size_t)L.first;

@@ -434,6 +434,49 @@ __device__ uint32_t light_samples(const ShadeView &sv, const Params &prm, const 
   return cnt;
 }
 
+// Of the BRDF samples [i0, i0 + n) of one vertex (n <= 32; sample i draws from the
+// sample index sidx0 + i, the first nlobe from the specular lobe, the rest cosine),
+// the ones whose direction may meet a light (MESH_ONLY: a mesh light): bit i - i0.  A
+// conservative test against each light's bounding sphere, about a tenth of the work of
+// the exact one: few of these directions meet a light (one in thirty on the box scene),
+// and the ones that do not add nothing.  A cosine direction is formed with the fast
+// sine, cosine and square root (within 2e-6 of sample_cosine's); the sphere is widened
+// by 2e-4 of its distance and its squared tangent length by 1e-5, well above that and
+// the rounding of these sums.  NaN counts as "may meet".
+template <bool MESH_ONLY>
+__device__ __forceinline__ uint32_t may_meet_light(const ShadeView &sv, const Surface &S, const Material &M,
+                                                   uint64_t key, uint32_t sample, uint32_t depth, F3 o_off,
+                                                   uint32_t sidx0, uint32_t i0, uint32_t n, uint32_t nlobe) {
+  const uint32_t all = n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+  F3 X, Y;
+  ref_frame(S.n, X, Y);
+  uint32_t mask = 0;
+  for (uint32_t k = 0; k < sv.first_point; ++k) {
+    const DevLight &L = sv.lights[k];
+    if (MESH_ONLY && L.type != CKR_LIGHT_MESH) continue;
+    const F3 l = f3(L.px, L.py, L.pz) - o_off;
+    const float ll = dot(l, l), rr = L.radius + 2e-4f * sqrtf(ll);
+    const float thr = ll - rr * rr - 1e-5f * ll;
+    if (!(thr > 0.f)) return all;  // inside or at the sphere
+    const float lx = dot(l, X), ly = dot(l, Y), ln = dot(l, S.n);
+    for (uint32_t j = 0; j < n; ++j) {
+      const float e1 = ckr_draw_f(key, ctr(sample, depth, 3 * (sidx0 + i0 + j) + 1));
+      const float e2 = ckr_draw_f(key, ctr(sample, depth, 3 * (sidx0 + i0 + j) + 2));
+      float b;
+      if (i0 + j < nlobe) {
+        b = dot(l, sample_lobe(M, S.n, S.wo_ref, S.wo, e1, e2));
+      } else {
+        float sp, cp;  // of 2 pi e2 - pi, inside the fast functions' accurate range
+        __sincosf(2.0f * kPi * (e2 - 0.5f), &sp, &cp);
+        const float st = e1 * rsqrtf(e1), ct = (1.0f - e1) * rsqrtf(1.0f - e1);
+        b = ct * ln - st * (cp * lx + sp * ly);
+      }
+      if (!(b < 0.f || b * b < thr)) mask |= 1u << j;
+    }
+  }
+  return mask;
+}
+
 // getLightAnalytic / getLightAnalyticDiffuse over every mesh light
 // (src/lightSources_CV.cpp:221-321): spec * amplitude * sum L |I_ltc| / 2pi +
 // (1 - spec) * sum L |I_cos| / 2pi.
@@ -631,30 +674,35 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
       F3 res = f3(0, 0, 0);
       const uint32_t nb = prm.n_brdf, nlobe = (uint32_t)((float)nb * M.spec);
       const uint32_t nls = sv.first_point * prm.n_light;
-      for (uint32_t si = 0; si < nls + nb; ++si) {
-        float e0 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si));
-        float e1 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 1));
-        float e2 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 2));
-        F3 w = si < nls ? sample_light(sv, sv.lights[si / prm.n_light], S.x, e0, e1, e2)
+      // A sample adds nothing unless its direction meets a mesh light: the BRDF samples
+      // are first cut down to those that may (may_meet_light), 32 at a time, and only
+      // these run the queries and the BRDF's terms (box, 512^2 x 4 spp, 10 light + 60
+      // BRDF samples: 4.83 -> 2.63 ms).  The sums' order stays the samples'.
+      for (uint32_t s0 = 0; s0 < nls + nb;) {
+        const bool lights = s0 < nls;
+        const uint32_t cnt = min(32u, (lights ? nls : nls + nb) - s0);
+        uint32_t todo = cnt >= 32 ? 0xffffffffu : (1u << cnt) - 1u;
+        if (!lights) todo = may_meet_light<true>(sv, S, M, key, meta.y, meta.z, o_off, nls, s0 - nls, cnt, nlobe);
+        while (todo) {
+          const uint32_t si = s0 + __ffs(todo) - 1;
+          todo &= todo - 1;
+          float e0 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si));
+          float e1 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 1));
+          float e2 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 2));
+          F3 w = lights ? sample_light(sv, sv.lights[si / prm.n_light], S.x, e0, e1, e2)
                         : (si - nls < nlobe ? sample_lobe(M, S.n, S.wo_ref, S.wo, e1, e2) : sample_cosine(S.n, e1, e2));
-        float c = dot(w, S.n);
-        if (c < 0.f) continue;
-        LightQuery lq = query_lights(sv, S.x, o_off, w, prm.n_light);
-        float denom = lq.pdf_sum + (float)nb * pdf_eval(M, S.n, S.wo_ref, S.wo, w);
-        // First mesh light in list order that the direction meets.
-        RayPre r = ray_pre(o_off, w, 0.f);
-        for (uint32_t k = 0; k < sv.nlights; ++k) {
-          DevLight L = sv.lights[k];
-          if (L.type != CKR_LIGHT_MESH) continue;
-          float t;
-          uint32_t id = light_tri_hit(sv, L, r, t);
-          if (id == kMiss) continue;
+          float c = dot(w, S.n);
+          if (c < 0.f) continue;
+          LightQuery lq = query_lights(sv, S.x, o_off, w, prm.n_light);
+          if (lq.mesh == kMiss) continue;
+          // lq.mesh: of the first mesh light in list order that the direction meets.
+          float denom = lq.pdf_sum + (float)nb * pdf_eval(M, S.n, S.wo_ref, S.wo, w);
           float fa = brdf_eval(M, S.n, S.wo_ref, S.wo, w) * sv.mats[S.mat].reflectance;
           float fl = (ltc_on ? brdf_ltc(M, Lk, minv, S.n, w) : brdf_eval(M, S.n, S.wo_ref, S.wo, w)) *
                      sv.mats[S.mat].reflectance;
-          res = res + mat_radiance(sv, sv.tri_mat[id]) * ((fa - fl) * c / (denom + 1e-20f));
-          break;
+          res = res + mat_radiance(sv, sv.tri_mat[lq.mesh]) * ((fa - fl) * c / (denom + 1e-20f));
         }
+        s0 += cnt;
       }
       const ckr_material &mm = sv.mats[S.mat];
       F3 col = f3(mm.color[0], mm.color[1], mm.color[2]);
