@@ -13,8 +13,8 @@
 // spp and depth share the grid until the last path has started.
 //
 // A path draws the same random numbers and runs the same device functions as in
-// the wavefront shaders (camera_ray, make_surface, light_samples, sample_brdf,
-// pdf_eval, brdf_eval, query_lights, select/nee_pdf, trace_ray), so each job's
+// the wavefront shaders (camera_ray, make_surface, technique_dir, sample_brdf,
+// brdf_pdf_eval, query_lights, select/nee_pdf, trace_ray), so each job's
 // image equals ckr_render of that job up to the order of the FP64 sums.
 #pragma once
 #include "wavefront.cuh"
@@ -25,6 +25,8 @@ namespace {
 // Shadow rays a vertex may need (lights x samples); larger batches use the
 // wavefront renderer.
 constexpr uint32_t kInlineShadow = 4;
+
+__device__ __forceinline__ float4 f4(F3 v) { return make_float4(v.x, v.y, v.z, 0.f); }
 
 struct LaneShadow {
   float4 o[kInlineShadow], d[kInlineShadow], c[kInlineShadow];
@@ -71,7 +73,26 @@ __device__ __noinline__ bool vertex_path(const ShadeView &sv0, const Params &prm
   const F3 fcol = f3(mm.color[0], mm.color[1], mm.color[2]) * mm.reflectance;
   const uint64_t key = ckr_key(pc.seed, meta.x - pc.px_base);
   const F3 o_off = offset_origin(S.x, S.n);
-  sh.n = light_samples<false, LF>(sv, prm, S, M, fcol, beta, key, meta.y, meta.z, o_off, sh.o, sh.d, sh.c, true);
+  for (uint32_t k = sv.first_point; (LF & kLightPoint) && k < sv.nlights; ++k) {
+    F3 contrib;
+    if (point_sample(sv.lights[k], S, M, fcol, beta, o_off, sh.d[sh.n], contrib)) sh.c[sh.n++] = f4(contrib);
+  }
+  const uint32_t nls = sv.first_point * prm.n_light, nlt = nls + ((LF & kLightEnv) ? sv.env_n : 0u);
+  for (uint32_t si = 0; si < nlt; ++si) {
+    const F3 wl = technique_dir<LF>(sv, prm, S.x, si, nls, ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si)),
+                                    ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 1)),
+                                    ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 2)));
+    const float cl = dot(wl, S.n);
+    if (cl < 0.f) continue;
+    const LightQuery ll = query_lights<true, LF>(sv, S.x, o_off, wl, prm.n_light);
+    if (!ll.hit) continue;
+    float fl, pl;
+    brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, wl, fl, pl);
+    const float denom = ll.pdf_sum + (float)prm.n_brdf * pl;
+    sh.d[sh.n] = make_float4(wl.x, wl.y, wl.z, shadow_tmax(ll.d));
+    sh.c[sh.n++] = f4(mulc(beta, mulc(fcol, ll.Le)) * (fl * cl / (denom + 1e-20f)));
+  }
+  for (uint32_t k = 0; k < sh.n; ++k) sh.o[k] = f4(o_off);
   const float e0 = ckr_draw_f(key, ctr(meta.y, meta.z, kDimBrdf));
   const float e1 = ckr_draw_f(key, ctr(meta.y, meta.z, kDimBrdf + 1));
   const float e2 = ckr_draw_f(key, ctr(meta.y, meta.z, kDimBrdf + 2));
@@ -79,8 +100,8 @@ __device__ __noinline__ bool vertex_path(const ShadeView &sv0, const Params &prm
   const float c = dot(w, S.n);
   const float err = ckr_draw_f(key, ctr(meta.y, meta.z, kDimRR));
   if (!(c > 0.f && err >= prm.rr_prob)) return false;
-  const float pb = pdf_eval(M, S.n, S.wo_ref, S.wo, w);
-  const float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
+  float f, pb;
+  brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, pb);
   if (!(pb > 0.f && f > 0.f)) return false;
   const LightQuery lq = query_lights<true, LF>(sv, S.x, o_off, w, prm.n_light);
   const float wb = (float)prm.n_brdf * pb / ((float)prm.n_brdf * pb + lq.pdf_sum);
@@ -159,9 +180,9 @@ __device__ __noinline__ bool vertex_nee(const ShadeView &sv0, const Params &prm,
     const float cl = fabsf(dot(nrm, w)) / len;
     if (c > 0.f && cl > 0.f && len > 0.f && dist > 0.f) {
       const float pl = nee_pdf(sv, select_prob(sv, none, j), L, tri, dist, 0.5f * len, cl);
-      const float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
+      float f, pb;
+      brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, pb);
       if (pl > 0.f && f > 0.f) {
-        const float pb = pdf_eval(M, S.n, S.wo_ref, S.wo, w);
         const F3 Le = mat_radiance(sv, sv.tri_mat[tri]);
         const float g = f * c / pl;
         const F3 contrib = mulc(beta, mulc(fcol, Le)) * (g * (pl / (pl + pb)));
@@ -181,8 +202,8 @@ __device__ __noinline__ bool vertex_nee(const ShadeView &sv0, const Params &prm,
   const float cn = dot(wn, S.n);
   const float err = ckr_draw_f(key, ctr(meta.y, meta.z, kDimRR));
   if (!(cn > 0.f && err >= prm.rr_prob)) return false;
-  const float pb = pdf_eval(M, S.n, S.wo_ref, S.wo, wn);
-  const float f = brdf_eval(M, S.n, S.wo_ref, S.wo, wn);
+  float f, pb;
+  brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, wn, f, pb);
   if (!(pb > 0.f && f > 0.f)) return false;
   const F3 nb = mulc(beta, fcol) * (f * cn / (pb * (1.0f - prm.rr_prob)));
   ro = make_float4(o_off.x, o_off.y, o_off.z, 0.f);

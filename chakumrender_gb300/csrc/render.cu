@@ -54,6 +54,37 @@ __global__ void k_tri_nm(const float *__restrict__ tri9, const uint32_t *__restr
   out[i] = make_float4(n.x, n.y, n.z, __uint_as_float(tri_mat[i]));
 }
 
+// The shading kernel of a render: one of three signatures.
+struct ShadeFn {
+  void (*lit)(ShadeView, Paths, Params, int, int, const LtcEntry *) = nullptr;  // PATH, DIRECT_MISCV
+  void (*trace)(ShadeView, Paths, Params, int, int, const LtcEntry *, SceneView, int) = nullptr;
+  void (*nee)(ShadeView, Paths, Params, int, Learn) = nullptr;
+  const void *fn() const { return lit ? (const void *)lit : trace ? (const void *)trace : (const void *)nee; }
+  void launch(int grid, size_t smem, cudaStream_t stream, const ShadeView &shv, const Paths &P, const Params &prm,
+              int cur, int d, const LtcEntry *ltc, const SceneView &sv, int stack_depth, const Learn &lr) const {
+    if (lit) lit<<<grid, kRTPB, smem, stream>>>(shv, P, prm, cur, d, ltc);
+    else if (trace) trace<<<grid, kRTPB, smem, stream>>>(shv, P, prm, cur, d, ltc, sv, stack_depth);
+    else nee<<<grid, kRTPB, smem, stream>>>(shv, P, prm, cur, lr);
+  }
+};
+
+// LF: without the code of light kinds the scene does not have.
+template <uint32_t LF>
+ShadeFn shade_fn_lf(uint32_t shader) {
+  ShadeFn f;
+  if (shader == CKR_SHADER_PATH_NEE) f.nee = k_shade_nee<kRTPB>;
+  else if (shader == CKR_SHADER_PATH) f.lit = k_shade_path<kRTPB, LF>;
+  else if (shader == CKR_SHADER_EXPLICIT) f.trace = k_shade<CKR_SHADER_EXPLICIT, kRTPB, LF>;
+  else if (shader == CKR_SHADER_DIRECT_CV) f.trace = k_shade<CKR_SHADER_DIRECT_CV, kRTPB, kLightsAll>;
+  else if (shader == CKR_SHADER_DIRECT_MIS) f.trace = k_shade<CKR_SHADER_DIRECT_MIS, kRTPB, LF>;
+  else f.lit = k_shade_miscv<kRTPB, LF>;
+  return f;
+}
+
+ShadeFn shade_fn_of(const ckr_scene *s, uint32_t shader) {
+  return mesh_lights_only(s) ? shade_fn_lf<kLightsMeshOnly>(shader) : shade_fn_lf<kLightsAll>(shader);
+}
+
 struct Workspace {
   DevBuf<float4> ray_o, ray_d, beta, sh_o, sh_d, sh_c;
   DevBuf<uint4> meta;
@@ -226,19 +257,10 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
   }
   const int g_ext = grid_for((const void *)extend_fn, smem, kRTPB);
   const int g_sh = grid_for((const void *)shadow_fn, smem, kRTPB);
+  const ShadeFn shade = shade_fn_of(s, cfg->shader);
   if (cfg->shader == CKR_SHADER_EXPLICIT && smem > 48 * 1024)
-    CKR_CUDA_TRY(cudaFuncSetAttribute(k_shade<CKR_SHADER_EXPLICIT, kRTPB>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // The path shader without the code of light kinds the scene does not have.
-  void (*const path_fn)(ShadeView, Paths, Params, int, int, const LtcEntry *) =
-      mesh_lights_only(s) ? k_shade_path<kRTPB, kLightsMeshOnly> : k_shade_path<kRTPB, kLightsAll>;
-  const void *shade_fn = cfg->shader == CKR_SHADER_EXPLICIT ? (const void *)k_shade<CKR_SHADER_EXPLICIT, kRTPB>
-                         : cfg->shader == CKR_SHADER_PATH_NEE ? (const void *)k_shade_nee<kRTPB>
-                         : cfg->shader == CKR_SHADER_PATH      ? (const void *)path_fn
-                         : cfg->shader == CKR_SHADER_DIRECT_CV  ? (const void *)k_shade<CKR_SHADER_DIRECT_CV, kRTPB>
-                         : cfg->shader == CKR_SHADER_DIRECT_MIS ? (const void *)k_shade<CKR_SHADER_DIRECT_MIS, kRTPB>
-                                                                : (const void *)k_shade_miscv<kRTPB>;
-  const int g_shade = grid_for(shade_fn, cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, kRTPB);
+    CKR_CUDA_TRY(cudaFuncSetAttribute(shade.fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int g_shade = grid_for(shade.fn(), cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, kRTPB);
   // One step of the wavefront over queue `cur`: closest hit, [learned selection],
   // shading, shadow rays, [training].  k: the step's index within the wave (or the
   // render, with regeneration) -- it picks the selection buffer, and k = 0 has no
@@ -292,18 +314,7 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
       }
     }
     const int d = (int)std::min<uint64_t>(k, prm.max_depth);
-    if (cfg->shader == CKR_SHADER_EXPLICIT)
-      k_shade<CKR_SHADER_EXPLICIT, kRTPB><<<g_shade, kRTPB, smem, stream>>>(shv, P, prm, cur, d, ltc, sv, depth);
-    else if (cfg->shader == CKR_SHADER_PATH_NEE)
-      k_shade_nee<kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, lr);
-    else if (cfg->shader == CKR_SHADER_PATH)
-      path_fn<<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, d, ltc);
-    else if (cfg->shader == CKR_SHADER_DIRECT_CV)
-      k_shade<CKR_SHADER_DIRECT_CV, kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, d, ltc);
-    else if (cfg->shader == CKR_SHADER_DIRECT_MIS)
-      k_shade<CKR_SHADER_DIRECT_MIS, kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, d, ltc);
-    else
-      k_shade_miscv<kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, d, ltc);
+    shade.launch(g_shade, cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, stream, shv, P, prm, cur, d, ltc, sv, depth, lr);
     shadow_fn<<<g_sh, kRTPB, smem, stream>>>(sv, P, depth, cur, train && nee ? rec : nullptr);
     if (train && nee) {
       // Adam steps on this step's light samples (visibility applied above),
@@ -625,19 +636,10 @@ extern "C" int ckr_render_noalloc(ckr_scene *s, const ckr_camera *cam, const ckr
   }
   const int g_ext = grid_for((const void *)extend_fn, smem, kRTPB);
   const int g_sh = grid_for((const void *)shadow_fn, smem, kRTPB);
+  const ShadeFn shade = shade_fn_of(s, cfg->shader);
   if (cfg->shader == CKR_SHADER_EXPLICIT && smem > 48 * 1024)
-    CKR_CUDA_TRY(cudaFuncSetAttribute(k_shade<CKR_SHADER_EXPLICIT, kRTPB>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // The path shader without the code of light kinds the scene does not have.
-  void (*const path_fn)(ShadeView, Paths, Params, int, int, const LtcEntry *) =
-      mesh_lights_only(s) ? k_shade_path<kRTPB, kLightsMeshOnly> : k_shade_path<kRTPB, kLightsAll>;
-  const void *shade_fn = cfg->shader == CKR_SHADER_EXPLICIT ? (const void *)k_shade<CKR_SHADER_EXPLICIT, kRTPB>
-                         : cfg->shader == CKR_SHADER_PATH_NEE ? (const void *)k_shade_nee<kRTPB>
-                         : cfg->shader == CKR_SHADER_PATH      ? (const void *)path_fn
-                         : cfg->shader == CKR_SHADER_DIRECT_CV  ? (const void *)k_shade<CKR_SHADER_DIRECT_CV, kRTPB>
-                         : cfg->shader == CKR_SHADER_DIRECT_MIS ? (const void *)k_shade<CKR_SHADER_DIRECT_MIS, kRTPB>
-                                                                : (const void *)k_shade_miscv<kRTPB>;
-  const int g_shade = grid_for(shade_fn, cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, kRTPB);
+    CKR_CUDA_TRY(cudaFuncSetAttribute(shade.fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int g_shade = grid_for(shade.fn(), cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, kRTPB);
   for (uint64_t base = 0; base < total; base += wave) {
     uint32_t n = (uint32_t)std::min<uint64_t>(wave, total - base);
     k_camera<kRTPB><<<std::min<int>(g_ext, ceil_div(n, kRTPB)), kRTPB, 0, stream>>>(c, P, prm, base, n);
@@ -648,19 +650,8 @@ extern "C" int ckr_render_noalloc(ckr_scene *s, const ckr_camera *cam, const ckr
       extend_fn<<<g_ext, kRTPB, smem, stream>>>(sv, P, cur, depth);
       CKR_CUDA_TRY(cudaMemsetAsync(P.counts + (cur ^ 1), 0, sizeof(uint32_t), stream));
       CKR_CUDA_TRY(cudaMemsetAsync(P.counts + 2, 0, sizeof(uint32_t), stream));
-      if (cfg->shader == CKR_SHADER_EXPLICIT)
-        k_shade<CKR_SHADER_EXPLICIT, kRTPB><<<g_shade, kRTPB, smem, stream>>>(shv, P, prm, cur, (int)d, ltc, sv,
-                                                                              depth);
-      else if (cfg->shader == CKR_SHADER_PATH_NEE)
-        k_shade_nee<kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, Learn{});
-      else if (cfg->shader == CKR_SHADER_PATH)
-        path_fn<<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, (int)d, ltc);
-      else if (cfg->shader == CKR_SHADER_DIRECT_CV)
-        k_shade<CKR_SHADER_DIRECT_CV, kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, (int)d, ltc);
-      else if (cfg->shader == CKR_SHADER_DIRECT_MIS)
-        k_shade<CKR_SHADER_DIRECT_MIS, kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, (int)d, ltc);
-      else
-        k_shade_miscv<kRTPB><<<g_shade, kRTPB, 0, stream>>>(shv, P, prm, cur, (int)d, ltc);
+      shade.launch(g_shade, cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, stream, shv, P, prm, cur, (int)d, ltc, sv,
+                   depth, Learn{});
       shadow_fn<<<g_sh, kRTPB, smem, stream>>>(sv, P, depth, cur, nullptr);
       cur ^= 1;
       if (!path) break;

@@ -176,6 +176,39 @@ SHD float pdf_eval(const Material &m, F3 n, F3 wo_ref, F3 wo, F3 wi) {
   return s + diffuse;
 }
 
+// brdf_eval and pdf_eval of one direction, with the half vector and the distribution
+// (its power or exponential) formed once and one copy of their code: the shading
+// kernels are bound by instruction fetch.  The same operations as the two functions.
+SHD void brdf_pdf_eval(const Material &m, F3 n, F3 wo_ref, F3 wo, F3 wi, float &f, float &p) {
+  const float diffuse = (1.0f - m.spec) * dot(wi, n) / kPi;
+  const float s = m.spec;
+  f = 0.0f;
+  p = s;
+  if (m.brdf == kClassicPhong) {
+    const float c = dot(wo_ref, wi);
+    const float e = powf(c > 0.f ? c : 0.f, m.phong_exp);
+    f = s * (m.phong_exp + 1.0f) * e / (2.0f * kPi) + (1.0f - s) / kPi;
+    p = s * ((m.phong_exp + 1.0f) * e / (2.0f * kPi));
+  } else if (m.brdf == kGGX || m.brdf == kBeckmann || m.brdf == kPhong) {
+    const F3 h = normalize(wo + wi);
+    const float F = fresnel(m, dot(h, wi));
+    float D, G;
+    if (m.brdf == kGGX) {
+      D = ggx_dist(m.alpha, h, n);
+      G = ggx_g1(m.alpha, wo, h, n) * ggx_g1(m.alpha, wi, h, n);
+    } else if (m.brdf == kBeckmann) {
+      D = beckmann_dist(m.alpha, h, n);
+      G = beckmann_g1(m.alpha, wo, h, n) * beckmann_g1(m.alpha, wi, h, n);
+    } else {
+      D = phong_dist(m.alpha, h, n);
+      G = phong_g1(m.alpha, wo, h, n) * phong_g1(m.alpha, wi, h, n);
+    }
+    f = (s * F * D * G) / (4.0f * dot(wi, n) * dot(wo, n)) + (1.0f - s) / kPi;
+    p = s * (D * dot(h, n) / (4.0f * dot(h, wo)));
+  }
+  p = p + diffuse;
+}
+
 // ---- samplers (src/domainSampler.cpp) ------------------------------------------
 // Tangent frame of the reference (src/domainSampler.cpp:163-176):
 // X = normalize((-n.y - n.z) / n.x, 1, 1) when n.x != 0, else
@@ -212,40 +245,39 @@ SHD F3 sample_hemisphere(F3 n, float e1, float e2) {
   return to_world(X, Y, n, st * cp, st * sp, ct);
 }
 
-// Specular lobe of getBrdfDirectionSamples / getClassicPhongDirectionSamples
-// (src/domainSampler.cpp:193-314).
-SHD F3 sample_lobe(const Material &m, F3 n, F3 wo_ref, F3 wo, float e1, float e2) {
-  float sp, cp;
-  sincosf(2.0f * kPi * e2, &sp, &cp);
+// One direction of the BRDF techniques: `lobe`, the specular lobe of
+// getBrdfDirectionSamples / getClassicPhongDirectionSamples
+// (src/domainSampler.cpp:193-314), else the cosine direction (sample_cosine).  One
+// copy of the frame, the sine and cosine and the power serves all of them.
+SHD F3 sample_dir(const Material &m, F3 n, F3 wo_ref, F3 wo, bool lobe, float e1, float e2) {
+  const bool classic = lobe && m.brdf == kClassicPhong;
+  const F3 Z = classic ? wo_ref : n;
   F3 X, Y;
-  if (m.brdf == kClassicPhong) {
-    ref_frame(wo_ref, X, Y);
-    float ct = powf(1.0f - e1, 1.0f / (m.phong_exp + 1.0f));
-    float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
-    return to_world(X, Y, wo_ref, st * cp, st * sp, ct);
-  }
-  ref_frame(n, X, Y);
+  ref_frame(Z, X, Y);
   float ct, st;
-  if (m.brdf == kGGX) {
-    float tt = m.alpha * sqrtf(e1) / sqrtf(1.0f - e1 + 1e-10f);
-    ct = 1.0f / sqrtf(1.0f + tt * tt);
-    st = tt * ct;
-  } else if (m.brdf == kBeckmann) {
-    float tt = sqrtf(-(m.alpha * m.alpha) * logf(1.0f - e1 + 1e-20f));
+  if (!lobe) {
+    st = sqrtf(e1);
+    ct = sqrtf(1.0f - e1);
+  } else if (m.brdf == kGGX || m.brdf == kBeckmann) {
+    const float tt = m.brdf == kGGX ? m.alpha * sqrtf(e1) / sqrtf(1.0f - e1 + 1e-10f)
+                                    : sqrtf(-(m.alpha * m.alpha) * logf(1.0f - e1 + 1e-20f));
     ct = 1.0f / sqrtf(1.0f + tt * tt);
     st = tt * ct;
   } else {
-    ct = powf(e1, 1.0f / (m.alpha + 2.0f));
+    ct = powf(classic ? 1.0f - e1 : e1, 1.0f / (classic ? m.phong_exp + 1.0f : m.alpha + 2.0f));
     st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
   }
-  F3 h = to_world(X, Y, n, st * cp, st * sp, ct);
+  float sp, cp;
+  sincosf(2.0f * kPi * e2, &sp, &cp);
+  const F3 h = to_world(X, Y, Z, st * cp, st * sp, ct);
+  if (!lobe || classic) return h;
   return normalize(h * (2.0f * dot(h, wo)) - wo);
 }
 
 // getBrdfDirectionSampleRandomized (src/materialTypes.cpp:136-153): the lobe with
 // probability spec, else cosine.
 SHD F3 sample_brdf(const Material &m, F3 n, F3 wo_ref, F3 wo, float e0, float e1, float e2) {
-  return e0 < m.spec ? sample_lobe(m, n, wo_ref, wo, e1, e2) : sample_cosine(n, e1, e2);
+  return sample_dir(m, n, wo_ref, wo, e0 < m.spec, e1, e2);
 }
 
 // Cone of half-angle theta_max about w (getSolidDirectionSamples,

@@ -75,17 +75,6 @@ struct Paths {
   int *status;       // the scene's device status word (first CKR_ERR_*)
 };
 
-// Shadow rays of one shading step past the queue's capacity are dropped and the
-// status word records CKR_ERR_QUEUE_OVERFLOW (the host sizes the queue so that
-// this cannot happen; the check keeps a wrong size from writing out of bounds).
-__device__ __forceinline__ uint32_t shadow_fit(const Paths &P, uint32_t sbase, uint32_t nshadow) {
-  if (nshadow && sbase + nshadow > P.sh_cap) {
-    atomicCAS(P.status, 0, CKR_ERR_QUEUE_OVERFLOW);
-    return 0;
-  }
-  return nshadow;
-}
-
 // One job of a batched render: its paths are the global path indices
 // [path_begin, path_begin + npix * spp), its pixels the accumulation rows
 // [accum_off, accum_off + npix), its materials sv.mats[mat_off ...].
@@ -150,20 +139,31 @@ __device__ __forceinline__ uint32_t job_of(const JobDev *jobs, uint32_t njobs, u
   return lo;
 }
 
-// Reserves `k` consecutive slots per lane in a queue; all 32 lanes must call.
-__device__ __forceinline__ uint32_t warp_reserve(uint32_t *counter, uint32_t k) {
-  const int lane = threadIdx.x & 31;
-  uint32_t incl = k;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += v;
-  }
-  uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+// One slot of a queue for each lane that wants one; all 32 lanes must call.
+__device__ __forceinline__ uint32_t ballot_reserve(uint32_t *counter, bool want) {
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  if (m == 0) return 0;
+  const uint32_t lane = threadIdx.x & 31u, leader = __ffs(m) - 1;
   uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(counter, total);
-  base = __shfl_sync(0xffffffffu, base, 31);
-  return base + incl - k;
+  if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
+  return __shfl_sync(0xffffffffu, base, leader) + __popc(m & ((1u << lane) - 1u));
+}
+
+// Appends one shadow ray for each lane that wants one; all 32 lanes must call.  Rays
+// past the queue's capacity are dropped and the status word records
+// CKR_ERR_QUEUE_OVERFLOW (the host sizes the queue so that this cannot happen; the
+// check keeps a wrong size from writing out of bounds).
+__device__ __forceinline__ void emit_shadow(const Paths &P, bool want, F3 o, float4 d, F3 contrib, uint32_t px) {
+  const uint32_t at = ballot_reserve(&P.counts[2], want);
+  if (!want) return;
+  if (at >= P.sh_cap) {
+    atomicCAS(P.status, 0, CKR_ERR_QUEUE_OVERFLOW);
+    return;
+  }
+  P.sh_o[at] = make_float4(o.x, o.y, o.z, 0.f);
+  P.sh_d[at] = d;
+  P.sh_c[at] = make_float4(contrib.x, contrib.y, contrib.z, 0.f);
+  P.sh_px[at] = px;
 }
 
 __device__ __forceinline__ void add_px(double *accum, uint32_t px, F3 c) {
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(TPB) k_camera(Cam cam0, Paths P, Params prm, u
 // slot now holds a fresh camera path.  All 32 lanes must call.
 __device__ __forceinline__ bool regenerate(const Params &prm, const Paths &P, bool ended, uint32_t slot) {
   if (!prm.regen_total) return false;
-  const uint32_t g = warp_reserve(&P.counts[5], ended ? 1u : 0u);
+  const uint32_t g = ballot_reserve(&P.counts[5], ended);
   if (!ended || g >= prm.regen_total) return false;
   camera_path(prm.cam, prm, P, g, slot);
   return true;
@@ -335,103 +335,31 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, 
     trace_static<true, TPB>(s, n, smem_trav + threadIdx.x, depth, fetch, finish);
 }
 
-// Light-technique samples at one surface: returns the number of shadow rays
-// written (one per sample whose direction meets a light), each with its
-// pre-weighted contribution  f * L * cos / sum_k N_k p_k.
-template <bool DETERMINISTIC_SPLIT, uint32_t LF = kLightsAll>
-__device__ uint32_t light_samples(const ShadeView &sv, const Params &prm, const Surface &S, const Material &M,
-                                  F3 fcol, F3 beta, uint64_t key, uint32_t sample, uint32_t depth, F3 o_off,
-                                  float4 *so, float4 *sd, float4 *sc, bool write) {
-  uint32_t cnt = 0, sidx = 0;
-  // Point lights: deterministic, no MIS (src/lightSources.cpp:48-63).
-  for (uint32_t k = sv.first_point; (LF & kLightPoint) && k < sv.nlights; ++k) {
-    DevLight L = sv.lights[k];
-    F3 dl = f3(L.px, L.py, L.pz) - S.x;
-    float dist = length(dl);
-    F3 w = dl * (1.0f / dist);
-    float c = dot(w, S.n);
-    if (c < 0.f) continue;
-    if (write) {
-      float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
-      float sc4 = c * f / (4.0f * kPi * dist * dist);
-      F3 contrib = mulc(beta, mulc(fcol, f3(L.pr, L.pg, L.pb))) * sc4;
-      so[cnt] = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
-      sd[cnt] = make_float4(w.x, w.y, w.z, shadow_tmax(length(f3(L.px, L.py, L.pz) - o_off)));
-      sc[cnt] = make_float4(contrib.x, contrib.y, contrib.z, 0.f);
-    }
-    ++cnt;
-  }
-  // Area and sphere lights: N samples each.  Lights are stored in the reference's
-  // getSamples order (sphere sources, mesh sources, triangle sources, then point
-  // lights; src/mis.cpp:100-146), so sample s belongs to light s / N.
-  for (uint32_t k = 0; k < sv.nlights; ++k) {
-    DevLight L = sv.lights[k];
-    if (L.type == CKR_LIGHT_POINT) break;
-    for (uint32_t i = 0; i < prm.n_light; ++i, ++sidx) {
-      float e0 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx));
-      float e1 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx + 1));
-      float e2 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx + 2));
-      F3 w = sample_light<LF>(sv, L, S.x, e0, e1, e2);
-      float c = dot(w, S.n);
-      if (c < 0.f) continue;
-      LightQuery lq = query_lights<true, LF>(sv, S.x, o_off, w, prm.n_light);
-      if (!lq.hit) continue;
-      if (write) {
-        float denom = lq.pdf_sum + (float)prm.n_brdf * pdf_eval(M, S.n, S.wo_ref, S.wo, w);
-        float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
-        F3 contrib = mulc(beta, mulc(fcol, lq.Le)) * (f * c / (denom + 1e-20f));
-        so[cnt] = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
-        sd[cnt] = make_float4(w.x, w.y, w.z, shadow_tmax(lq.d));
-        sc[cnt] = make_float4(contrib.x, contrib.y, contrib.z, 0.f);
-      }
-      ++cnt;
-    }
-  }
-  // Environment light: its own technique after the area lights (EnMpIS of
-  // MIS::getSamples, src/mis.cpp:154-166).
-  for (uint32_t i = 0; (LF & kLightEnv) && i < sv.env_n; ++i, ++sidx) {
-    float e0 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx));
-    float e1 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx + 1));
-    float e2 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx + 2));
-    F3 w = env_sample(sv, e0, e1, e2);
-    float c = dot(w, S.n);
-    if (c < 0.f) continue;
-    LightQuery lq = query_lights<true, LF>(sv, S.x, o_off, w, prm.n_light);
-    if (!lq.hit) continue;
-    if (write) {
-      float denom = lq.pdf_sum + (float)prm.n_brdf * pdf_eval(M, S.n, S.wo_ref, S.wo, w);
-      float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
-      F3 contrib = mulc(beta, mulc(fcol, lq.Le)) * (f * c / (denom + 1e-20f));
-      so[cnt] = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
-      sd[cnt] = make_float4(w.x, w.y, w.z, shadow_tmax(lq.d));
-      sc[cnt] = make_float4(contrib.x, contrib.y, contrib.z, 0.f);
-    }
-    ++cnt;
-  }
-  if (DETERMINISTIC_SPLIT) {
-    // BRDF technique of MIS::getSamples: N*spec lobe samples, the rest cosine
-    // (MaterialType::getBrdfDirectionSamples, src/materialTypes.cpp:118-134).
-    uint32_t nb = prm.n_brdf, nlobe = (uint32_t)((float)nb * M.spec);
-    for (uint32_t i = 0; i < nb; ++i, ++sidx) {
-      float e1 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx + 1));
-      float e2 = ckr_draw_f(key, ctr(sample, depth, 3 * sidx + 2));
-      F3 w = i < nlobe ? sample_lobe(M, S.n, S.wo_ref, S.wo, e1, e2) : sample_cosine(S.n, e1, e2);
-      float c = dot(w, S.n);
-      if (c < 0.f) continue;
-      LightQuery lq = query_lights<true, LF>(sv, S.x, o_off, w, prm.n_light);
-      if (!lq.hit) continue;
-      if (write) {
-        float denom = lq.pdf_sum + (float)nb * pdf_eval(M, S.n, S.wo_ref, S.wo, w);
-        float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
-        F3 contrib = mulc(beta, mulc(fcol, lq.Le)) * (f * c / (denom + 1e-20f));
-        so[cnt] = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
-        sd[cnt] = make_float4(w.x, w.y, w.z, shadow_tmax(lq.d));
-        sc[cnt] = make_float4(contrib.x, contrib.y, contrib.z, 0.f);
-      }
-      ++cnt;
-    }
-  }
-  return cnt;
+// The sample of point light L (deterministic, no MIS, src/lightSources.cpp:48-63):
+// false below the surface, else the shadow ray's direction and tmax and its contribution.
+__device__ __forceinline__ bool point_sample(const DevLight &L, const Surface &S, const Material &M, F3 fcol, F3 beta,
+                                             F3 o_off, float4 &d4, F3 &contrib) {
+  F3 dl = f3(L.px, L.py, L.pz) - S.x;
+  float dist = length(dl);
+  F3 w = dl * (1.0f / dist);
+  float c = dot(w, S.n);
+  if (c < 0.f) return false;
+  float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
+  float sc4 = c * f / (4.0f * kPi * dist * dist);
+  contrib = mulc(beta, mulc(fcol, f3(L.pr, L.pg, L.pb))) * sc4;
+  d4 = make_float4(w.x, w.y, w.z, shadow_tmax(length(f3(L.px, L.py, L.pz) - o_off)));
+  return true;
+}
+
+// Direction of the light techniques' sample si of one vertex: n_light samples per
+// area and sphere light (lights are stored in the reference's getSamples order, sphere
+// sources, mesh sources, triangle sources; src/mis.cpp:100-146, so sample si belongs
+// to light si / n_light), then the environment's (EnMpIS, src/mis.cpp:154-166).
+template <uint32_t LF>
+__device__ __forceinline__ F3 technique_dir(const ShadeView &sv, const Params &prm, F3 x, uint32_t si, uint32_t nls,
+                                            float e0, float e1, float e2) {
+  if ((LF & kLightEnv) && si >= nls) return env_sample(sv, e0, e1, e2);
+  return sample_light<LF>(sv, sv.lights[si / prm.n_light], x, e0, e1, e2);
 }
 
 // Of the BRDF samples [i0, i0 + n) of one vertex (n <= 32; sample i draws from the
@@ -464,7 +392,7 @@ __device__ __forceinline__ uint32_t may_meet_light(const ShadeView &sv, const Su
       const float e2 = ckr_draw_f(key, ctr(sample, depth, 3 * (sidx0 + i0 + j) + 2));
       float b;
       if (i0 + j < nlobe) {
-        b = dot(l, sample_lobe(M, S.n, S.wo_ref, S.wo, e1, e2));
+        b = dot(l, sample_dir(M, S.n, S.wo_ref, S.wo, true, e1, e2));
       } else {
         float sp, cp;  // of 2 pi e2 - pi, inside the fast functions' accurate range
         __sincosf(2.0f * kPi * (e2 - 0.5f), &sp, &cp);
@@ -505,54 +433,54 @@ __device__ __forceinline__ F3 ltc_term(const ShadeView &sv, const Surface &S, co
 // The sampled part of getLightFromMeshSource_AnalyticCV (src/lightSources_CV.cpp:335-397):
 // per mesh light, n_light points by MeshLight::getSamples (300-bin CDF, sqrt(u1)
 // barycentrics), each adding Le (V f - f_ltc) cos cos_l / d^2 * area / n.  The
-// unoccluded -f_ltc part is summed into `neg`; each +f part is a shadow ray whose
-// contribution is returned through so/sd/sc when WRITE.  Returns the ray count.
-template <bool WRITE>
-__device__ uint32_t cv_samples(const ShadeView &sv, const Params &prm, const Surface &S, const Material &M, float refl,
-                               const LtcLookup &Lk, const M3f &minv, bool ltc_on, F3 col, uint64_t key,
-                               uint32_t sample, F3 o_off, F3 &neg, float4 *so, float4 *sd, float4 *sc) {
-  uint32_t cnt = 0, sidx = 0;
+// unoccluded -f_ltc part is summed into `neg`; each +f part is a shadow ray.  All 32
+// lanes must call (`surface`: this lane has a vertex).
+__device__ __forceinline__ void cv_samples(const ShadeView &sv, const Paths &P, const Params &prm, bool surface,
+                                           const Surface &S, const Material &M, const LtcLookup &Lk, const M3f &minv,
+                                           bool ltc_on, uint64_t key, const uint4 &meta, F3 o_off, F3 &neg) {
+  uint32_t sidx = 0;
   for (uint32_t k = 0; k < sv.first_point; ++k) {
     DevLight L = sv.lights[k];
     if (L.type != CKR_LIGHT_MESH) continue;
     const float w_area = L.area / (float)prm.n_light;
     for (uint32_t i = 0; i < prm.n_light; ++i, ++sidx) {
-      float e0 = ckr_draw_f(key, ctr(sample, 0, 3 * sidx));
-      float e1 = ckr_draw_f(key, ctr(sample, 0, 3 * sidx + 1));
-      float e2 = ckr_draw_f(key, ctr(sample, 0, 3 * sidx + 2));
-      uint32_t b = (uint32_t)(e0 * (float)kInvCdfBins);
-      b = b >= kInvCdfBins ? kInvCdfBins - 1 : b;
-      const uint32_t tri = L.first + __ldg(&sv.cdf[L.cdf + b]);
-      const float *t9 = sv.tri9 + 9 * (size_t)tri;
-      F3 A = f3(__ldg(t9), __ldg(t9 + 1), __ldg(t9 + 2));
-      F3 B = f3(__ldg(t9 + 3), __ldg(t9 + 4), __ldg(t9 + 5));
-      F3 C = f3(__ldg(t9 + 6), __ldg(t9 + 7), __ldg(t9 + 8));
-      F3 Pl = sample_triangle(A, B, C, e1, e2);
-      F3 dv = Pl - S.x;
-      float d2 = dot(dv, dv), d = sqrtf(d2);
-      F3 w = dv * (1.0f / d);
-      float c = dot(w, S.n);
-      if (c < 0.f) continue;
-      float c1 = fabsf(dot(w, tri_normal(sv, tri)));
-      float g = c * c1 / d2 * w_area;
-      F3 Le = mat_radiance(sv, sv.tri_mat[tri]);
-      float fa = brdf_eval(M, S.n, S.wo_ref, S.wo, w) * refl;
-      if (!WRITE) {
-        float fl = (ltc_on ? brdf_ltc(M, Lk, minv, S.n, w) : brdf_eval(M, S.n, S.wo_ref, S.wo, w)) * refl;
-        neg = neg - Le * (fl * g);
-      }
-      if (fa > 0.f) {
-        if (WRITE) {
-          F3 contrib = mulc(col, Le) * (fa * g);
-          so[cnt] = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
-          sd[cnt] = shadow_dir(o_off, Pl);
-          sc[cnt] = make_float4(contrib.x, contrib.y, contrib.z, 0.f);
+      bool want = false;
+      float4 d4 = make_float4(0, 0, 0, 0);
+      F3 contrib = f3(0, 0, 0);
+      if (surface) {
+        float e0 = ckr_draw_f(key, ctr(meta.y, 0, 3 * sidx));
+        float e1 = ckr_draw_f(key, ctr(meta.y, 0, 3 * sidx + 1));
+        float e2 = ckr_draw_f(key, ctr(meta.y, 0, 3 * sidx + 2));
+        uint32_t b = (uint32_t)(e0 * (float)kInvCdfBins);
+        b = b >= kInvCdfBins ? kInvCdfBins - 1 : b;
+        const uint32_t tri = L.first + __ldg(&sv.cdf[L.cdf + b]);
+        const float *t9 = sv.tri9 + 9 * (size_t)tri;
+        F3 A = f3(__ldg(t9), __ldg(t9 + 1), __ldg(t9 + 2));
+        F3 B = f3(__ldg(t9 + 3), __ldg(t9 + 4), __ldg(t9 + 5));
+        F3 C = f3(__ldg(t9 + 6), __ldg(t9 + 7), __ldg(t9 + 8));
+        F3 Pl = sample_triangle(A, B, C, e1, e2);
+        F3 dv = Pl - S.x;
+        float d2 = dot(dv, dv), d = sqrtf(d2);
+        F3 w = dv * (1.0f / d);
+        float c = dot(w, S.n);
+        if (!(c < 0.f)) {
+          float c1 = fabsf(dot(w, tri_normal(sv, tri)));
+          float g = c * c1 / d2 * w_area;
+          F3 Le = mat_radiance(sv, sv.tri_mat[tri]);
+          const ckr_material &mm = sv.mats[S.mat];
+          float fa = brdf_eval(M, S.n, S.wo_ref, S.wo, w) * mm.reflectance;
+          float fl = ltc_on ? brdf_ltc(M, Lk, minv, S.n, w) * mm.reflectance : fa;
+          neg = neg - Le * (fl * g);
+          if (fa > 0.f) {
+            want = true;
+            contrib = mulc(f3(mm.color[0], mm.color[1], mm.color[2]), Le) * (fa * g);
+            d4 = shadow_dir(o_off, Pl);
+          }
         }
-        ++cnt;
       }
+      emit_shadow(P, want, o_off, d4, contrib, meta.x);
     }
   }
-  return cnt;
 }
 
 // Continuation dims of CKR_SHADER_EXPLICIT: RR at kDimRR, redraws r < kExplicitTries
@@ -572,7 +500,6 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
     uint32_t i = base + lane;
     bool valid = i < n;
     uint32_t slot = valid ? q[i] : 0;
-    uint32_t nshadow = 0;
     bool cont = false;
     float4 next_d = make_float4(0, 0, 0, 0), next_b = make_float4(0, 0, 0, 0);
     F3 next_o = f3(0, 0, 0);
@@ -625,7 +552,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
         }
       }
     }
-    // ---- direct light: count the shadow rays, reserve, then write them ----
+    // ---- direct light ----
     LtcLookup Lk{};
     M3f minv{};
     bool ltc_on = false;
@@ -638,26 +565,74 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
       minv = ltc_minv_world(Lk, S.n, S.wo);
       ltc_on = M.brdf == kGGX || M.brdf == kGGXApprox;
     }
-    if (surface && SHADER == CKR_SHADER_DIRECT_CV)
-      nshadow = cv_samples<false>(sv, prm, S, M, sv.mats[S.mat].reflectance, Lk, minv, ltc_on,
-                                  f3(sv.mats[S.mat].color[0], sv.mats[S.mat].color[1], sv.mats[S.mat].color[2]), key,
-                                  meta.y, o_off, cv_neg, nullptr, nullptr, nullptr);
-    else if (surface && SHADER != CKR_SHADER_DIRECT_MISCV && SHADER != CKR_SHADER_EXPLICIT)
-      nshadow = light_samples<SHADER == CKR_SHADER_DIRECT_MIS, LF>(sv, prm, S, M, fcol, beta, key, meta.y, meta.z,
-                                                                   o_off, nullptr, nullptr, nullptr, false);
-    uint32_t sbase = warp_reserve(&P.counts[2], nshadow);
-    nshadow = shadow_fit(P, sbase, nshadow);
-    if (nshadow) {
-      if (SHADER == CKR_SHADER_DIRECT_CV) {
-        F3 unused = f3(0, 0, 0);
-        cv_samples<true>(sv, prm, S, M, sv.mats[S.mat].reflectance, Lk, minv, ltc_on,
-                         f3(sv.mats[S.mat].color[0], sv.mats[S.mat].color[1], sv.mats[S.mat].color[2]), key, meta.y,
-                         o_off, unused, P.sh_o + sbase, P.sh_d + sbase, P.sh_c + sbase);
-      } else {
-        light_samples<SHADER == CKR_SHADER_DIRECT_MIS, LF>(sv, prm, S, M, fcol, beta, key, meta.y, meta.z, o_off,
-                                                       P.sh_o + sbase, P.sh_d + sbase, P.sh_c + sbase, true);
+    if (SHADER == CKR_SHADER_DIRECT_CV)
+      cv_samples(sv, P, prm, surface, S, M, Lk, minv, ltc_on, key, meta, o_off, cv_neg);
+    if (SHADER == CKR_SHADER_PATH || SHADER == CKR_SHADER_DIRECT_MIS) {
+      // Point lights, then the MIS set: the light techniques' samples, and the BRDF
+      // samples (DIRECT_MIS, N * spec lobe samples, the rest cosine, as
+      // getBrdfDirectionSamples, src/materialTypes.cpp:118-134) or the one BRDF sample
+      // that continues the path (PATH).  A light's, the environment's and a BRDF sample
+      // all take the same query and BRDF evaluation, one copy of their code in one loop,
+      // and a sample's shadow ray is appended as soon as it is known (counting the rays
+      // first and forming them in a second pass took every sample twice: box path frame
+      // 1.049 -> 0.927 ms, small-batch pass 3.52 -> 3.03 ms).  The loop is the same for all lanes of a warp, and every lane
+      // takes part in its reservations.
+      for (uint32_t k = sv.first_point; (LF & kLightPoint) && k < sv.nlights; ++k) {
+        float4 d4 = make_float4(0, 0, 0, 0);
+        F3 contrib = f3(0, 0, 0);
+        const bool want = surface && point_sample(sv.lights[k], S, M, fcol, beta, o_off, d4, contrib);
+        emit_shadow(P, want, o_off, d4, contrib, meta.x);
       }
-      for (uint32_t k = 0; k < nshadow; ++k) P.sh_px[sbase + k] = meta.x;
+      const uint32_t nls = sv.first_point * prm.n_light, nlt = nls + ((LF & kLightEnv) ? sv.env_n : 0u);
+      const uint32_t nb = SHADER == CKR_SHADER_PATH ? 1u : prm.n_brdf;
+      const uint32_t nlobe = surface ? (uint32_t)((float)nb * M.spec) : 0u;
+      for (uint32_t s0 = 0; s0 < nlt + nb;) {
+        const bool light = s0 < nlt, last = SHADER == CKR_SHADER_PATH && !light;
+        const uint32_t cnt = min(32u, (light ? nlt : nlt + nb) - s0);
+        uint32_t todo = !surface ? 0u : cnt >= 32 ? 0xffffffffu : (1u << cnt) - 1u;
+        // BRDF samples that meet no light add nothing (with an environment all do).
+        if (SHADER == CKR_SHADER_DIRECT_MIS && surface && !light && !((LF & kLightEnv) && sv.env_n))
+          todo = may_meet_light<false>(sv, S, M, key, meta.y, meta.z, o_off, nlt, s0 - nlt, cnt, nlobe);
+        while (__any_sync(0xffffffffu, todo)) {
+          bool want = false;
+          float4 d4 = make_float4(0, 0, 0, 0);
+          F3 contrib = f3(0, 0, 0);
+          if (todo) {
+            const uint32_t si = s0 + __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t dim = last ? kDimBrdf : 3 * si;
+            const float e0 = ckr_draw_f(key, ctr(meta.y, meta.z, dim));
+            const float e1 = ckr_draw_f(key, ctr(meta.y, meta.z, dim + 1));
+            const float e2 = ckr_draw_f(key, ctr(meta.y, meta.z, dim + 2));
+            const F3 w = light ? technique_dir<LF>(sv, prm, S.x, si, nls, e0, e1, e2)
+                               : sample_dir(M, S.n, S.wo_ref, S.wo,
+                                            SHADER == CKR_SHADER_PATH ? e0 < M.spec : si - nlt < nlobe, e1, e2);
+            const float c = dot(w, S.n);
+            if (last ? c > 0.f && ckr_draw_f(key, ctr(meta.y, meta.z, kDimRR)) >= prm.rr_prob : !(c < 0.f)) {
+              const LightQuery lq = query_lights<true, LF>(sv, S.x, o_off, w, prm.n_light);
+              if (last || lq.hit) {
+                float f, p;
+                brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, p);
+                if (!last) {
+                  const float denom = lq.pdf_sum + (float)nb * p;
+                  contrib = mulc(beta, mulc(fcol, lq.Le)) * (f * c / (denom + 1e-20f));
+                  d4 = make_float4(w.x, w.y, w.z, shadow_tmax(lq.d));
+                  want = true;
+                } else if (p > 0.f && f > 0.f) {
+                  const float wb = (float)nb * p / ((float)nb * p + lq.pdf_sum);
+                  const F3 nbeta = mulc(beta, fcol) * (f * c / (p * (1.0f - prm.rr_prob)));
+                  cont = true;
+                  next_o = o_off;
+                  next_d = make_float4(w.x, w.y, w.z, 3.0e38f);
+                  next_b = make_float4(nbeta.x, nbeta.y, nbeta.z, wb);
+                }
+              }
+            }
+          }
+          if (!last) emit_shadow(P, want, o_off, d4, contrib, meta.x);
+        }
+        s0 += cnt;
+      }
     }
     if (surface && SHADER == CKR_SHADER_DIRECT_CV) {
       // getLightFromMeshSource_AnalyticCV: the LTC term plus the unoccluded part of
@@ -677,7 +652,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
       // A sample adds nothing unless its direction meets a mesh light: the BRDF samples
       // are first cut down to those that may (may_meet_light), 32 at a time, and only
       // these run the queries and the BRDF's terms (box, 512^2 x 4 spp, 10 light + 60
-      // BRDF samples: 4.83 -> 2.63 ms).  The sums' order stays the samples'.
+      // BRDF samples: 4.84 -> 2.63 ms).  The sums' order stays the samples'.
       for (uint32_t s0 = 0; s0 < nls + nb;) {
         const bool lights = s0 < nls;
         const uint32_t cnt = min(32u, (lights ? nls : nls + nb) - s0);
@@ -689,17 +664,18 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
           float e0 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si));
           float e1 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 1));
           float e2 = ckr_draw_f(key, ctr(meta.y, meta.z, 3 * si + 2));
-          F3 w = lights ? sample_light(sv, sv.lights[si / prm.n_light], S.x, e0, e1, e2)
-                        : (si - nls < nlobe ? sample_lobe(M, S.n, S.wo_ref, S.wo, e1, e2) : sample_cosine(S.n, e1, e2));
+          F3 w = lights ? sample_light<LF>(sv, sv.lights[si / prm.n_light], S.x, e0, e1, e2)
+                        : sample_dir(M, S.n, S.wo_ref, S.wo, si - nls < nlobe, e1, e2);
           float c = dot(w, S.n);
           if (c < 0.f) continue;
-          LightQuery lq = query_lights(sv, S.x, o_off, w, prm.n_light);
+          LightQuery lq = query_lights<false, LF>(sv, S.x, o_off, w, prm.n_light);
           if (lq.mesh == kMiss) continue;
           // lq.mesh: of the first mesh light in list order that the direction meets.
-          float denom = lq.pdf_sum + (float)nb * pdf_eval(M, S.n, S.wo_ref, S.wo, w);
-          float fa = brdf_eval(M, S.n, S.wo_ref, S.wo, w) * sv.mats[S.mat].reflectance;
-          float fl = (ltc_on ? brdf_ltc(M, Lk, minv, S.n, w) : brdf_eval(M, S.n, S.wo_ref, S.wo, w)) *
-                     sv.mats[S.mat].reflectance;
+          float f, p;
+          brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, p);
+          float denom = lq.pdf_sum + (float)nb * p;
+          float fa = f * sv.mats[S.mat].reflectance;
+          float fl = ltc_on ? brdf_ltc(M, Lk, minv, S.n, w) * sv.mats[S.mat].reflectance : fa;
           res = res + mat_radiance(sv, sv.tri_mat[lq.mesh]) * ((fa - fl) * c / (denom + 1e-20f));
         }
         s0 += cnt;
@@ -751,30 +727,8 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
         P.hit_t[slot] = th;
       }
     }
-    // ---- continuation (path tracer) ----
-    if (surface && SHADER == CKR_SHADER_PATH) {
-      float e0 = ckr_draw_f(key, ctr(meta.y, meta.z, kDimBrdf));
-      float e1 = ckr_draw_f(key, ctr(meta.y, meta.z, kDimBrdf + 1));
-      float e2 = ckr_draw_f(key, ctr(meta.y, meta.z, kDimBrdf + 2));
-      F3 w = sample_brdf(M, S.n, S.wo_ref, S.wo, e0, e1, e2);
-      float c = dot(w, S.n);
-      float err = ckr_draw_f(key, ctr(meta.y, meta.z, kDimRR));
-      if (c > 0.f && err >= prm.rr_prob) {
-        float pb = pdf_eval(M, S.n, S.wo_ref, S.wo, w);
-        float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
-        if (pb > 0.f && f > 0.f) {
-          LightQuery lq = query_lights<true, LF>(sv, S.x, o_off, w, prm.n_light);
-          float wb = (float)prm.n_brdf * pb / ((float)prm.n_brdf * pb + lq.pdf_sum);
-          F3 nb = mulc(beta, fcol) * (f * c / (pb * (1.0f - prm.rr_prob)));
-          cont = true;
-          next_o = o_off;
-          next_d = make_float4(w.x, w.y, w.z, 3.0e38f);
-          next_b = make_float4(nb.x, nb.y, nb.z, wb);
-        }
-      }
-    }
     const bool fresh = regenerate(prm, P, valid && !cont, slot);
-    uint32_t cbase = warp_reserve(&P.counts[cur ^ 1], cont || fresh ? 1u : 0u);
+    uint32_t cbase = ballot_reserve(&P.counts[cur ^ 1], cont || fresh);
     if (cont) {
       // Continue in place: the path keeps its slot.  tmin = -1 marks a ray the
       // explicit loop has traced already.
@@ -800,11 +754,11 @@ constexpr int shade_blocks(uint32_t shader, int tpb) {
   return shader == CKR_SHADER_EXPLICIT ? (512 / tpb > 1 ? 512 / tpb : 1) : (1024 / tpb > 1 ? 1024 / tpb : 1);
 }
 
-template <uint32_t SHADER, int TPB>
+template <uint32_t SHADER, int TPB, uint32_t LF = kLightsAll>
 __global__ void __launch_bounds__(TPB, shade_blocks(SHADER, TPB)) k_shade(ShadeView sv0, Paths P, Params prm, int cur, int depth,
                                                  const LtcEntry *__restrict__ ltc, SceneView scene = SceneView{},
                                                  int stack_depth = 0) {
-  shade<SHADER, TPB>(sv0, P, prm, cur, depth, ltc, scene, stack_depth);
+  shade<SHADER, TPB, LF>(sv0, P, prm, cur, depth, ltc, scene, stack_depth);
 }
 
 // LF: the light kinds compiled in (kLightsMeshOnly for scenes whose lights are all
@@ -828,10 +782,10 @@ inline bool mesh_lights_only(const ckr_scene *s) {
 // registers at 128 threads, with spills): box, 512^2 x 4 spp, 10 light + 60 BRDF
 // samples: 6.13 ms at 512 / TPB (128 registers), 6.24 at 640, 5.89 at 768, 5.51 at
 // 1024, 5.83 at 1280, 5.78 at 1536; at 154 spill-free registers it was slower still.
-template <int TPB>
+template <int TPB, uint32_t LF = kLightsAll>
 __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
     k_shade_miscv(ShadeView sv0, Paths P, Params prm, int cur, int depth, const LtcEntry *__restrict__ ltc) {
-  shade<CKR_SHADER_DIRECT_MISCV, TPB>(sv0, P, prm, cur, depth, ltc, SceneView{}, 0);
+  shade<CKR_SHADER_DIRECT_MISCV, TPB, LF>(sv0, P, prm, cur, depth, ltc, SceneView{}, 0);
 }
 
 // CKR_SHADER_PATH_NEE: one light sample and one BRDF sample per vertex over many
@@ -926,9 +880,9 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
           float cl = fabsf(dot(nrm, w)) / len;
           if (c > 0.f && cl > 0.f && len > 0.f && dist > 0.f) {
             float pl = nee_pdf(sv, select_prob(sv, sel, j), L, tri, dist, 0.5f * len, cl);
-            float f = brdf_eval(M, S.n, S.wo_ref, S.wo, w);
+            float f, pb;
+            brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, pb);
             if (pl > 0.f && f > 0.f) {
-              float pb = pdf_eval(M, S.n, S.wo_ref, S.wo, w);
               F3 Le = mat_radiance(sv, sv.tri_mat[tri]);
               float g = f * c / pl;
               F3 contrib = mulc(beta, mulc(fcol, Le)) * (g * (pl / (pl + pb)));
@@ -956,8 +910,8 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
             float cn = dot(wn, S.n);
             float err = ckr_draw_f(key, ctr(meta.y, meta.z, kDimRR));
             if (cn > 0.f && err >= prm.rr_prob) {
-              float pb = pdf_eval(M, S.n, S.wo_ref, S.wo, wn);
-              float f = brdf_eval(M, S.n, S.wo_ref, S.wo, wn);
+              float f, pb;
+              brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, wn, f, pb);
               if (pb > 0.f && f > 0.f) {
                 F3 nb = mulc(beta, fcol) * (f * cn / (pb * (1.0f - prm.rr_prob)));
                 cont = true;
@@ -972,7 +926,7 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
     }
     uint32_t rbase = kNoRec;
     if (lr.rec) {
-      rbase = warp_reserve(lr.rec_count, rec_ok ? 1u : 0u);
+      rbase = ballot_reserve(lr.rec_count, rec_ok);
       if (rec_ok && rbase < lr.rec_cap) {
         lr.rec[3 * (size_t)rbase] = r0;
         lr.rec[3 * (size_t)rbase + 1] = r1;
@@ -981,9 +935,10 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
         rbase = kNoRec;
       }
     }
-    uint32_t sbase = warp_reserve(&P.counts[2], nshadow);
-    nshadow = shadow_fit(P, sbase, nshadow);
-    if (nshadow) {
+    const uint32_t sbase = ballot_reserve(&P.counts[2], nshadow != 0);
+    if (nshadow && sbase >= P.sh_cap) {
+      atomicCAS(P.status, 0, CKR_ERR_QUEUE_OVERFLOW);
+    } else if (nshadow) {
       P.sh_o[sbase] = so;
       P.sh_d[sbase] = sd;
       P.sh_c[sbase] = sc;
@@ -991,7 +946,7 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
       if (lr.rec) P.sh_rec[sbase] = rbase;
     }
     const bool fresh = regenerate(prm, P, valid && !cont, slot);
-    uint32_t cbase = warp_reserve(&P.counts[cur ^ 1], cont || fresh ? 1u : 0u);
+    uint32_t cbase = ballot_reserve(&P.counts[cur ^ 1], cont || fresh);
     if (cont) {
       P.ray_o[slot] = make_float4(next_o.x, next_o.y, next_o.z, 0.f);
       P.ray_d[slot] = next_d;
