@@ -162,12 +162,11 @@ int enqueue(ckr_batch *b, JobSet &set, bool pack, size_t wave, cudaStream_t stre
   ckr_scene *s = b->scene;
   const int depth = (int)stack_depth_of(s);
   size_t smem = (size_t)depth * TPB * sizeof(uint2);
-  smem += shear_smem_bytes(TPB);  // the triangle test's ray data (dynamic fetching)
   // Deep trees: dynamic fetching; one or two levels: one ray per thread.
-  const bool dyn = s->max_depth >= kDynamicDepth;
-  void (*const extend_fn)(SceneView, Paths, int, int) = dyn ? k_extend<TPB, true> : k_extend<TPB, false>;
-  void (*const shadow_fn)(SceneView, Paths, int, int, float4 *) =
-      dyn ? k_shadow<TPB, true> : k_shadow<TPB, false>;
+  const bool dyn = walk_of(s) != kWalkStatic;
+  if (dyn) smem += shear_smem_bytes(TPB);  // the triangle test's ray data
+  const ExtendFn extend_fn = extend_fn_of<TPB>(s);
+  const ShadowFn shadow_fn = shadow_fn_of<TPB>(s);
   if (smem > 48 * 1024) {
     CKR_CUDA_TRY(cudaFuncSetAttribute(extend_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CKR_CUDA_TRY(cudaFuncSetAttribute(shadow_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -245,12 +245,11 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
   ShadeView shv = shade_view_of(s);
   int depth = (int)stack_depth_of(s);
   size_t smem = (size_t)depth * kRTPB * sizeof(uint2);
-  smem += shear_smem_bytes(kRTPB);  // the triangle test's ray data (dynamic fetching)
   // Deep trees: dynamic fetching; one or two levels: one ray per thread.
-  const bool dyn = s->max_depth >= kDynamicDepth;
-  void (*const extend_fn)(SceneView, Paths, int, int) = dyn ? k_extend<kRTPB, true> : k_extend<kRTPB, false>;
-  void (*const shadow_fn)(SceneView, Paths, int, int, float4 *) =
-      dyn ? k_shadow<kRTPB, true> : k_shadow<kRTPB, false>;
+  const bool dyn = walk_of(s) != kWalkStatic;
+  if (dyn) smem += shear_smem_bytes(kRTPB);  // the triangle test's ray data
+  const ExtendFn extend_fn = extend_fn_of<kRTPB>(s);
+  const ShadowFn shadow_fn = shadow_fn_of<kRTPB>(s);
   if (smem > 48 * 1024) {
     CKR_CUDA_TRY(cudaFuncSetAttribute(extend_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CKR_CUDA_TRY(cudaFuncSetAttribute(shadow_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -624,12 +623,11 @@ extern "C" int ckr_render_noalloc(ckr_scene *s, const ckr_camera *cam, const ckr
   const LtcEntry *ltc = g_noalloc_ltc_dev[dev];
   int depth = (int)stack_depth_of(s);
   size_t smem = (size_t)depth * kRTPB * sizeof(uint2);
-  smem += shear_smem_bytes(kRTPB);  // the triangle test's ray data (dynamic fetching)
   // Deep trees: dynamic fetching; one or two levels: one ray per thread.
-  const bool dyn = s->max_depth >= kDynamicDepth;
-  void (*const extend_fn)(SceneView, Paths, int, int) = dyn ? k_extend<kRTPB, true> : k_extend<kRTPB, false>;
-  void (*const shadow_fn)(SceneView, Paths, int, int, float4 *) =
-      dyn ? k_shadow<kRTPB, true> : k_shadow<kRTPB, false>;
+  const bool dyn = walk_of(s) != kWalkStatic;
+  if (dyn) smem += shear_smem_bytes(kRTPB);  // the triangle test's ray data
+  const ExtendFn extend_fn = extend_fn_of<kRTPB>(s);
+  const ShadowFn shadow_fn = shadow_fn_of<kRTPB>(s);
   if (smem > 48 * 1024) {
     CKR_CUDA_TRY(cudaFuncSetAttribute(extend_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CKR_CUDA_TRY(cudaFuncSetAttribute(shadow_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

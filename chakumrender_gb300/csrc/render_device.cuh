@@ -236,9 +236,9 @@ __device__ __forceinline__ LightQuery query_lights(const ShadeView &sv, F3 x, F3
       float s = L.radius / len;
       float cmax = sqrtf(fmaxf(0.f, 1.0f - s * s));
       if (dot(w, wl * (1.0f / len)) >= cmax) q.pdf_sum += (float)n_per_light / (2.0f * kPi * (1.0f - cmax));
-      double ts = hit_sphere(r, make_float4(L.px, L.py, L.pz, L.radius));
-      if (ts < 1e299 && (float)ts < q.d) {
-        q.d = (float)ts;
+      const SphereRoot ts = hit_sphere(r, make_float4(L.px, L.py, L.pz, L.radius));
+      if (ts.code == 1 && ts.t < q.d) {
+        q.d = ts.t;
         q.Le = mat_radiance(sv, sv.sph_mat[L.first]);
         q.hit = true;
       }

@@ -48,14 +48,14 @@ constexpr int kTPB = 128;
 constexpr size_t kAfterStacksBytes = shear_smem_bytes(kTPB) + kSlotLutBytes;
 
 // Closest / any hit over a ray array, with dynamic ray fetching (trace_dynamic).
-template <bool ANY>
+template <bool ANY, bool SPHERES>
 __global__ void __launch_bounds__(kTPB) k_trace_dyn(SceneView s, const float4 *__restrict__ rays, uint32_t n,
                                                     uint32_t *__restrict__ hit_id, float *__restrict__ hit_t,
                                                     uint8_t *__restrict__ occluded, int depth, uint32_t *next) {
   extern __shared__ uint2 smem_trav[];
   float4 *col = shear_column<kTPB>(smem_trav, depth);
   const uint8_t *lut = fill_slot_lut<kTPB>(reinterpret_cast<uint8_t *>(col - threadIdx.x + 3 * kTPB));
-  const TriShearSmem<kTPB, true, true> tri_pol{col, lut};
+  const TriShearSmem<kTPB, true, true, SPHERES> tri_pol{col, lut};
   trace_dynamic<ANY>(
       s, n, next, smem_trav + threadIdx.x, kTPB, depth,
       [&](uint32_t i, RayPre &r, float &tmax) {
@@ -76,6 +76,14 @@ __global__ void __launch_bounds__(kTPB) k_trace_dyn(SceneView s, const float4 *_
       tri_pol);
 }
 
+using TraceFn = void (*)(SceneView, const float4 *, uint32_t, uint32_t *, float *, uint8_t *, int, uint32_t *);
+
+// The traversal kernel for scene s.
+template <bool ANY>
+TraceFn trace_fn(const ckr_scene *s) {
+  return s->nsph ? k_trace_dyn<ANY, true> : k_trace_dyn<ANY, false>;
+}
+
 struct LaunchShape {
   int grid;
   size_t smem;
@@ -92,10 +100,10 @@ cudaError_t launch_shape(const ckr_scene *s, LaunchShape &ls) {
   if (e != cudaSuccess) return e;
   ls.smem = (size_t)stack_depth_of(s) * kTPB * sizeof(uint2) + kAfterStacksBytes;
   if (ls.smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(k_trace_dyn<ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ls.smem);
+    e = cudaFuncSetAttribute(trace_fn<ANY>(s), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ls.smem);
     if (e != cudaSuccess) return e;
   }
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_dyn<ANY>, kTPB, ls.smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_fn<ANY>(s), kTPB, ls.smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   ls.grid = sms * per_sm;
@@ -113,7 +121,7 @@ int launch_trace(const ckr_scene *s, const ckr_ray *rays, uint32_t n, uint32_t *
   const size_t smem = s->trace_smem;
   // The attribute is per kernel: set it for this scene's stack before each launch.
   if (smem > 48 * 1024)
-    CKR_CUDA_TRY(cudaFuncSetAttribute(k_trace_dyn<ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CKR_CUDA_TRY(cudaFuncSetAttribute(trace_fn<ANY>(s), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // Launches cover at most 2^31 rays so that the counter, which overshoots n by at
   // most one refill per warp, cannot wrap.
   const bool own = next == nullptr;
@@ -124,7 +132,7 @@ int launch_trace(const ckr_scene *s, const ckr_ray *rays, uint32_t n, uint32_t *
     const uint32_t m = std::min(n - off, kChunk);
     e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) break;
-    k_trace_dyn<ANY><<<grid, kTPB, smem, stream>>>(
+    trace_fn<ANY>(s)<<<grid, kTPB, smem, stream>>>(
         view_of(s), reinterpret_cast<const float4 *>(rays + off), m, ANY ? nullptr : hit_id + off,
         ANY ? nullptr : hit_t + off, ANY ? occluded + off : nullptr, (int)stack_depth_of(s), next);
     e = cudaGetLastError();

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sphere_pair.h"
+
 namespace ckr {
 
 constexpr int32_t kDone = (int32_t)0x80000000;  // also the root link of an empty tree
@@ -138,52 +140,43 @@ __device__ __forceinline__ bool hit_triangle_sheared(const RayPre &r, const Shea
   return true;
 }
 
-// Sphere::intersect in FP64 (src/geometryPrimitives.cpp:12-27), with the
-// root taken above max(tmin, 1e-4).
+// Sphere::intersect (src/geometryPrimitives.cpp:12-27), with the root taken above
+// max(tmin, 1e-4): the FP64 test's answer, found without FP64 wherever FP32 can show it
+// (two pre-tests for misses, then the root in pairs of FP32 numbers, sphere_pair.h).
+// FP64 runs at 1.6 lanes per clock and SM here.
 // LEAVING: also the second pre-test, for rays leaving the sphere.  The traversal
 // kernels with dynamic fetching leave it out: their scenes here have no spheres, and
 // the extra code in their refill path cost 0.7 % (many-light frame, A/B).
 template <bool LEAVING = true>
-__device__ __forceinline__ double hit_sphere(const RayPre &r, float4 s) {
-  {
-    // FP32 pre-tests (FP64 is slow on this part).  A ray whose line passes the sphere
-    // by more than 1e-5 of the squared magnitudes involved -- orders of magnitude
-    // above the FP32 rounding of these few operations -- has a negative FP64
-    // discriminant too, so the miss is decided without FP64.  The rounding of b =
-    // (c - o).d grows with |d|, so the bound scales the (c - o) terms by
-    // max(1, |d|^2): directions need not have unit length.  NaN and overflow fall
-    // through to the FP64 test.
-    const float ox = s.x - r.ox, oy = s.y - r.oy, oz = s.z - r.oz;
-    const float b = ox * r.dx + oy * r.dy + oz * r.dz;
-    const float oo = ox * ox + oy * oy + oz * oz;
-    const float dd = fmaxf(1.f, r.dx * r.dx + r.dy * r.dy + r.dz * r.dz);
-    const float m = fmaxf(fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fabsf(s.z)),
-                          fmaxf(fmaxf(fabsf(r.ox), fabsf(r.oy)), fabsf(r.oz)));
-    const float T = (m * m + oo) * dd + b * b + s.w * s.w;
-    const float det = b * b - oo + s.w * s.w;
-    if (det < -1e-5f * T) return 1e300;
-    // A ray leaving the sphere (bounce and shadow rays from its surface, rays moving
-    // away from it): the far root b + sqrt(det) is below 5e-5 even with b and det
-    // raised by bounds on their FP32 rounding (4e-6 sqrt(T) and 4e-6 T, several times
-    // the few-ulp errors of these sums), so both roots are below the 1e-4 the FP64 test
-    // requires and it would report a miss.  NaN fails the comparison.
-    if constexpr (LEAVING) {
-      const float t2u = (b + 4e-6f * sqrtf(T)) + sqrtf(fmaxf(0.f, det + 4e-6f * T));
-      if (t2u < 5e-5f) return 1e300;
-    }
+__device__ __forceinline__ SphereRoot hit_sphere(const RayPre &r, float4 s) {
+  // FP32 pre-tests.  A ray whose line passes the sphere
+  // by more than 1e-5 of the squared magnitudes involved -- orders of magnitude
+  // above the FP32 rounding of these few operations -- has a negative FP64
+  // discriminant too, so the miss is decided at once.  The rounding of b =
+  // (c - o).d grows with |d|, so the bound scales the (c - o) terms by
+  // max(1, |d|^2): directions need not have unit length.  NaN and overflow fall
+  // through to the FP64 test.
+  const float ox = s.x - r.ox, oy = s.y - r.oy, oz = s.z - r.oz;
+  const float b = ox * r.dx + oy * r.dy + oz * r.dz;
+  const float oo = ox * ox + oy * oy + oz * oz;
+  const float dd = fmaxf(1.f, r.dx * r.dx + r.dy * r.dy + r.dz * r.dz);
+  const float m = fmaxf(fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fabsf(s.z)),
+                        fmaxf(fmaxf(fabsf(r.ox), fabsf(r.oy)), fabsf(r.oz)));
+  const float T = (m * m + oo) * dd + b * b + s.w * s.w;
+  const float det = b * b - oo + s.w * s.w;
+  if (det < -1e-5f * T) return SphereRoot{0.f, 0.f, 0};
+  // A ray leaving the sphere (bounce and shadow rays from its surface, rays moving
+  // away from it): the far root b + sqrt(det) is below 5e-5 even with b and det
+  // raised by bounds on their FP32 rounding (4e-6 sqrt(T) and 4e-6 T, several times
+  // the few-ulp errors of these sums), so both roots are below the 1e-4 the FP64 test
+  // requires and it would report a miss.  NaN fails the comparison.
+  if constexpr (LEAVING) {
+    const float t2u = (b + 4e-6f * sqrtf(T)) + sqrtf(fmaxf(0.f, det + 4e-6f * T));
+    if (t2u < 5e-5f) return SphereRoot{0.f, 0.f, 0};
   }
-  double opx = (double)s.x - r.ox, opy = (double)s.y - r.oy, opz = (double)s.z - r.oz;
-  double dx = r.dx, dy = r.dy, dz = r.dz;
-  double b = opx * dx + opy * dy + opz * dz;
-  double rr = (double)s.w;
-  double det = b * b - (opx * opx + opy * opy + opz * opz) + rr * rr;
-  if (det < 0.0) return 1e300;
-  det = sqrt(det);
-  double eps = fmax(1e-4, (double)r.tmin);
-  double t = b - det;
-  if (t > eps) return t;
-  t = b + det;
-  return t > eps ? t : 1e300;
+  const SphereRoot q = sphere_root_pair(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, s.x, s.y, s.z, s.w, r.tmin, T);
+  if (q.code != 2) return q;
+  return sphere_root_f64(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, s.x, s.y, s.z, s.w, r.tmin);
 }
 
 // Slack of the quantised slab test, 4 u (u = 2^-24).  The entry distance of a
@@ -338,6 +331,7 @@ struct TriInRegs {
   static constexpr bool kPermutePlanes = false;
   static constexpr bool kSlotBits = false;
   static constexpr bool kSphereLeaving = true;
+  static constexpr bool kSpheres = true;
   const uint8_t *lut = nullptr;
   __device__ __forceinline__ bool operator()(const RayPre &r, float4 v0, float4 v1, float4 v2, float tbest,
                                              float &t) const {
@@ -403,9 +397,10 @@ template <bool LEAVING = true>
 __device__ __forceinline__ bool trace_spheres_rt(const SceneView &s, const RayPre &r, float &tbest, uint32_t &best,
                                                  const bool ANY) {
   for (uint32_t k = 0; k < s.nsph; ++k) {
-    double t = hit_sphere<LEAVING>(r, __ldg(&s.spheres[k]));
-    if (t < (double)tbest) {
-      tbest = (float)t;
+    const SphereRoot h = hit_sphere<LEAVING>(r, __ldg(&s.spheres[k]));
+    // The unrounded root is below tbest.
+    if (h.code == 1 && (h.t < tbest || (h.t == tbest && h.rem < 0.f))) {
+      tbest = h.t;
       best = kSphereBit | k;
       if (ANY) return false;
     }
@@ -497,8 +492,11 @@ __device__ __forceinline__ const uint8_t *fill_slot_lut(uint8_t *lut) {
   return lut;
 }
 
-template <int TPB, bool PERMUTE, bool SLOTBITS = false>
+// SPHERES: the scene has spheres; without them their code stays out of the refill path
+// (with it, closest hit over 2^23 rays and no sphere took 2.156 ms instead of 2.06).
+template <int TPB, bool PERMUTE, bool SLOTBITS, bool SPHERES>
 struct TriShearSmem {
+  static constexpr bool kSpheres = SPHERES;
   static constexpr bool kPermutePlanes = PERMUTE;
   static constexpr bool kSlotBits = SLOTBITS;
   static constexpr bool kSphereLeaving = false;
@@ -534,7 +532,8 @@ __device__ __forceinline__ void trace_dynamic(const SceneView &s, uint32_t n, ui
         if (idx < n && fetch(idx, r, tbest)) {
           best = kMiss;
           st = trav_start(s, r);
-          live = trace_spheres_rt<Tri::kSphereLeaving>(s, r, tbest, best, ANY);
+          live = true;
+          if constexpr (Tri::kSpheres) live = trace_spheres_rt<Tri::kSphereLeaving>(s, r, tbest, best, ANY);
           active = true;
         }
       }

@@ -13,6 +13,7 @@
 #include "../../include/ckr.h"
 #include "../../include/ckr_test.h"
 #include "bvh_build.h"
+#include "sphere_pair.h"
 
 namespace ckr {
 void scene_host_arrays(const ckr_scene *s, const uint32_t **nodes, const float **tris, const float **spheres,
@@ -251,6 +252,27 @@ extern "C" int ckr_internal_replay(const float *tri9, uint32_t ntri, uint32_t ma
 // digest of the flattened tree (nodes, then triangle records) and its node count,
 // so that builds on different numbers of threads can be compared.  Not part of the
 // public ABI.
+extern "C" int ckr_internal_sphere_roots_host(const float *row, uint32_t n, int mode, float *t, float *rem,
+                                              int32_t *code) {
+  if (n && (!row || !t || !rem || !code)) return CKR_ERR_INVALID_ARGUMENT;
+  for (uint32_t i = 0; i < n; ++i, row += 11) {
+    const float ox = row[6] - row[0], oy = row[7] - row[1], oz = row[8] - row[2];
+    const float b = ox * row[3] + oy * row[4] + oz * row[5], oo = ox * ox + oy * oy + oz * oz;
+    const float dd = std::max(1.f, row[3] * row[3] + row[4] * row[4] + row[5] * row[5]);
+    float m = 0.f;
+    for (int k : {0, 1, 2, 6, 7, 8}) m = std::max(m, std::fabs(row[k]));
+    const float T = (m * m + oo) * dd + b * b + row[9] * row[9];
+    const ckr::SphereRoot q =
+        mode ? ckr::sphere_root_f64(row[0], row[1], row[2], row[3], row[4], row[5], row[6], row[7], row[8], row[9], row[10])
+             : ckr::sphere_root_pair(row[0], row[1], row[2], row[3], row[4], row[5], row[6], row[7], row[8], row[9],
+                                     row[10], T);
+    t[i] = q.t;
+    rem[i] = q.rem;
+    code[i] = q.code;
+  }
+  return CKR_OK;
+}
+
 extern "C" int ckr_internal_bvh_digest(const float *tri9, uint32_t ntri, uint32_t max_leaf, uint32_t threads,
                                        uint64_t *digest, uint32_t *nnodes) {
   if (!digest || !nnodes) return CKR_ERR_INVALID_ARGUMENT;

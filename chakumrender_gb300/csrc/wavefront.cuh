@@ -23,6 +23,7 @@
 #include "ckr_internal.h"
 #include "ltc_table.h"
 #include "render_device.cuh"
+#include "scene.h"
 
 namespace ckr {
 namespace {
@@ -253,6 +254,10 @@ __device__ __forceinline__ bool regenerate(const Params &prm, const Paths &P, bo
 // scene (eight levels), 960x540 x 16 spp: 26.3 ms static, 23.0 ms dynamic.
 constexpr uint32_t kDynamicDepth = 3;
 
+// How k_extend / k_shadow walk the tree: one ray per thread, or dynamic fetching with
+// or without the scene's spheres.
+enum Walk : int { kWalkStatic = 0, kWalkDyn = 1, kWalkDynNoSpheres = 2 };
+
 // Resident blocks of k_extend / k_shadow: 1024 / TPB, i.e. 64 registers.  One ray
 // per thread (shallow trees): box frame 1.233 -> 1.208 ms against the compiler's
 // choice.  Dynamic fetching (deep trees), where the triangle test's ray data (shear
@@ -263,9 +268,9 @@ constexpr uint32_t kDynamicDepth = 3;
 // box test keeps the conversion form (the permute form at eight CTAs: 0.301 s).
 constexpr int trace_blocks(int tpb) { return 1024 / tpb < 1 ? 1 : 1024 / tpb; }
 
-// Closest hit of the paths in queue `cur`.  DYN: dynamic fetching over the queue,
-// work counter P.counts[3] (zeroed before the launch).
-template <int TPB, bool DYN>
+// Closest hit of the paths in queue `cur`.  Dynamic fetching over the queue takes its
+// work from the counter P.counts[3] (zeroed before the launch).
+template <int TPB, Walk WALK>
 __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_extend(SceneView s, Paths P, int cur, int depth) {
   extern __shared__ uint2 smem_trav[];
   const uint32_t *q = cur ? P.q1 : P.q0;
@@ -282,7 +287,7 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_extend(SceneView s, 
     P.hit_id[slot] = best;
     P.hit_t[slot] = t;
   };
-  if (DYN) {
+  if constexpr (WALK != kWalkStatic) {
     float4 *col = shear_column<TPB>(smem_trav, depth);
     auto fetch_s = [&](uint32_t i, RayPre &r, float &tmax) {
       if (!fetch(i, r, tmax)) return false;
@@ -290,15 +295,15 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_extend(SceneView s, 
       return true;
     };
     trace_dynamic<false>(s, P.counts[cur], P.counts + 3, smem_trav + threadIdx.x, TPB, depth, fetch_s, finish,
-                         TriShearSmem<TPB, false>{col});
+                         TriShearSmem<TPB, false, false, WALK == kWalkDyn>{col});
   } else
     trace_static<false, TPB>(s, P.counts[cur], smem_trav + threadIdx.x, depth, fetch, finish);
 }
 
 // Any hit of the shadow queue: unoccluded rays add their contribution to the
-// pixel; occluded ones zero their training record's weight.  DYN: dynamic
-// fetching, work counter P.counts[4] (zeroed before the launch).
-template <int TPB, bool DYN>
+// pixel; occluded ones zero their training record's weight.  Dynamic
+// fetching takes its work from the counter P.counts[4] (zeroed before the launch).
+template <int TPB, Walk WALK>
 __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, Paths P, int depth, int cur, float4 *rec) {
   extern __shared__ uint2 smem_trav[];
   const uint32_t n = min(P.counts[2], P.sh_cap);
@@ -322,7 +327,7 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, 
       if (ri != kNoRec) rec[3 * (size_t)ri + 1].w = 0.f;  // occluded: the sample contributed nothing
     }
   };
-  if (DYN) {
+  if constexpr (WALK != kWalkStatic) {
     float4 *col = shear_column<TPB>(smem_trav, depth);
     auto fetch_s = [&](uint32_t i, RayPre &r, float &tmax) {
       fetch(i, r, tmax);
@@ -330,9 +335,29 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, 
       return true;
     };
     trace_dynamic<true>(s, n, P.counts + 4, smem_trav + threadIdx.x, TPB, depth, fetch_s, finish,
-                        TriShearSmem<TPB, false>{col});
+                        TriShearSmem<TPB, false, false, WALK == kWalkDyn>{col});
   } else
     trace_static<true, TPB>(s, n, smem_trav + threadIdx.x, depth, fetch, finish);
+}
+
+using ExtendFn = void (*)(SceneView, Paths, int, int);
+using ShadowFn = void (*)(SceneView, Paths, int, int, float4 *);
+inline Walk walk_of(const ckr_scene *s) {
+  return s->max_depth < kDynamicDepth ? kWalkStatic : s->nsph ? kWalkDyn : kWalkDynNoSpheres;
+}
+template <int TPB>
+ExtendFn extend_fn_of(const ckr_scene *s) {
+  const Walk w = walk_of(s);
+  return w == kWalkStatic ? k_extend<TPB, kWalkStatic>
+         : w == kWalkDyn  ? k_extend<TPB, kWalkDyn>
+                          : k_extend<TPB, kWalkDynNoSpheres>;
+}
+template <int TPB>
+ShadowFn shadow_fn_of(const ckr_scene *s) {
+  const Walk w = walk_of(s);
+  return w == kWalkStatic ? k_shadow<TPB, kWalkStatic>
+         : w == kWalkDyn  ? k_shadow<TPB, kWalkDyn>
+                          : k_shadow<TPB, kWalkDynNoSpheres>;
 }
 
 // The sample of point light L (deterministic, no MIS, src/lightSources.cpp:48-63):

@@ -39,6 +39,10 @@ int ckr_internal_ltc_shade_host(const float *gbuf, uint32_t npx, const float *li
  * theta_over_sin) on the host, per value. */
 int ckr_internal_theta_over_sin_host(const float *c, uint32_t n, float *out);
 
+/* The sphere roots the kernels use, on the host, per row of (ox oy oz dx dy dz cx cy cz
+ * r tmin): mode 0 the pairs of FP32 numbers (code 0 miss, 1 hit, 2 undecided), 1 FP64. */
+int ckr_internal_sphere_roots_host(const float *row11, uint32_t n, int mode, float *t, float *rem, int32_t *code);
+
 /* The network's loss and gradients on n 12-float records in device memory,
  * computed by the tensor-core training kernels without an Adam step. */
 int ckr_internal_proposal_gradients(ckr_proposal *p, const float *rec12, uint32_t n, float *grad, float *loss);
