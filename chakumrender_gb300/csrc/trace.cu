@@ -307,7 +307,10 @@ int trace_host(ckr_scene *s, const ckr_ray *rays, uint32_t n, uint32_t *hit_id, 
   // end); the results are still staged and copied back chunk by chunk.
   const bool in_place = aligned16(rays) && device_addressable(rays, (size_t)n * sizeof(ckr_ray));
   const uint32_t chunk = kHostChunk;
-  uint32_t cap = (uint32_t)std::min<uint64_t>(n, (uint64_t)kPipes * chunk);
+  // Each stream's staging slot holds its largest chunk; chunks start at chunk / 8 when
+  // rays are uploaded, so a call of fewer than `chunk` rays can use every slot.
+  const uint32_t slot_cap = std::min(n, chunk), first_size = in_place ? chunk : chunk >> 3;
+  const uint32_t cap = n <= first_size ? n : kPipes * slot_cap;
   if (!in_place) CKR_CUDA_TRY(s->st_rays.reserve(cap));
   CKR_CUDA_TRY(s->st_next.reserve(kPipes));
   if (ANY) {
@@ -328,13 +331,13 @@ int trace_host(ckr_scene *s, const ckr_ray *rays, uint32_t n, uint32_t *hit_id, 
   // nothing overlaps, is short (e2e 3088 -> 3118 Mrays/s; shrinking the last chunks
   // as well was slower, 3035).
   // Rays read in place have no first upload to hide: full chunks from the start.
-  uint32_t k = 0, size = in_place ? chunk : chunk >> 3;
+  uint32_t k = 0, size = first_size;
   for (uint32_t off = 0; off < n; ++k) {
     const uint32_t m = std::min(size, n - off);
     size = std::min(size * 2, chunk);
     int slot = (int)(k % kPipes);
     cudaStream_t st = s->pipe[slot];
-    size_t base = (size_t)slot * chunk;
+    size_t base = (size_t)slot * slot_cap;
     if (!in_place)
       CKR_CUDA_TRY(cudaMemcpyAsync(s->st_rays.ptr + base, rays + off, (size_t)m * sizeof(ckr_ray),
                                    cudaMemcpyHostToDevice, st));
