@@ -48,40 +48,44 @@ constexpr int kTPB = 128;
 constexpr size_t kAfterStacksBytes = shear_smem_bytes(kTPB) + kSlotLutBytes;
 
 // Closest / any hit over a ray array, with dynamic ray fetching (trace_dynamic).
-template <bool ANY, bool SPHERES>
+template <bool ANY, bool SPHERES, bool DEALT>
 __global__ void __launch_bounds__(kTPB) k_trace_dyn(SceneView s, const float4 *__restrict__ rays, uint32_t n,
                                                     uint32_t *__restrict__ hit_id, float *__restrict__ hit_t,
-                                                    uint8_t *__restrict__ occluded, int depth, uint32_t *next) {
+                                                    uint8_t *__restrict__ occluded, int depth, uint32_t *next,
+                                                    uint32_t lanes) {
   extern __shared__ uint2 smem_trav[];
   float4 *col = shear_column<kTPB>(smem_trav, depth);
   const uint8_t *lut = fill_slot_lut<kTPB>(reinterpret_cast<uint8_t *>(col - threadIdx.x + 3 * kTPB));
   const TriShearSmem<kTPB, true, true, SPHERES> tri_pol{col, lut};
-  trace_dynamic<ANY>(
-      s, n, next, smem_trav + threadIdx.x, kTPB, depth,
-      [&](uint32_t i, RayPre &r, float &tmax) {
-        const float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
-        r = make_ray(a, b);
-        tmax = b.w;
-        store_shear<kTPB>(col, r);
-        return true;
-      },
-      [&](uint32_t i, uint32_t best, float t) {
-        if (ANY) {
-          occluded[i] = best != kMiss ? 1 : 0;
-        } else {
-          hit_id[i] = best;
-          hit_t[i] = t;
-        }
-      },
-      tri_pol);
+  auto fetch = [&](uint32_t i, RayPre &r, float &tmax) {
+    const float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
+    r = make_ray(a, b);
+    tmax = b.w;
+    store_shear<kTPB>(col, r);
+    return true;
+  };
+  auto finish = [&](uint32_t i, uint32_t best, float t) {
+    if (ANY) {
+      occluded[i] = best != kMiss ? 1 : 0;
+    } else {
+      hit_id[i] = best;
+      hit_t[i] = t;
+    }
+  };
+  if constexpr (DEALT)
+    trace_dealt<ANY>(s, n, lanes, smem_trav + threadIdx.x, kTPB, depth, fetch, finish, tri_pol);
+  else
+    trace_dynamic<ANY>(s, n, next, smem_trav + threadIdx.x, kTPB, depth, fetch, finish, tri_pol);
 }
 
-using TraceFn = void (*)(SceneView, const float4 *, uint32_t, uint32_t *, float *, uint8_t *, int, uint32_t *);
+using TraceFn = void (*)(SceneView, const float4 *, uint32_t, uint32_t *, float *, uint8_t *, int, uint32_t *,
+                         uint32_t);
 
-// The traversal kernel for scene s.
+// The traversal kernel for scene s (dealt: the launch deals the rays out, dealt_lanes).
 template <bool ANY>
-TraceFn trace_fn(const ckr_scene *s) {
-  return s->nsph ? k_trace_dyn<ANY, true> : k_trace_dyn<ANY, false>;
+TraceFn trace_fn(const ckr_scene *s, bool dealt) {
+  if (dealt) return s->nsph ? k_trace_dyn<ANY, true, true> : k_trace_dyn<ANY, false, true>;
+  return s->nsph ? k_trace_dyn<ANY, true, false> : k_trace_dyn<ANY, false, false>;
 }
 
 struct LaunchShape {
@@ -100,41 +104,105 @@ cudaError_t launch_shape(const ckr_scene *s, LaunchShape &ls) {
   if (e != cudaSuccess) return e;
   ls.smem = (size_t)stack_depth_of(s) * kTPB * sizeof(uint2) + kAfterStacksBytes;
   if (ls.smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(trace_fn<ANY>(s), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ls.smem);
+    e = cudaFuncSetAttribute(trace_fn<ANY>(s, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ls.smem);
     if (e != cudaSuccess) return e;
   }
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_fn<ANY>(s), kTPB, ls.smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_fn<ANY>(s, false), kTPB, ls.smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   ls.grid = sms * per_sm;
   return cudaSuccess;
 }
 
+// The pool the ray counters come from, one per device while that device has scenes.  The
+// device's default pool gives its memory back at every synchronisation, and mapping it
+// again took 180 us of a query that followed one (400,000 rays on 1,280 triangles: 288 us alone, 104 us
+// with this pool and the launches without a counter); this one keeps its single block
+// until the last scene goes.
+struct CounterPool {
+  std::mutex mu;
+  cudaMemPool_t pool[64] = {};
+  int refs[64] = {};
+};
+CounterPool &counter_pool() {
+  static CounterPool *p = new CounterPool();  // not destroyed: scenes may outlive static destruction
+  return *p;
+}
+
+// A reference for scene s (released by its destructor's caller); no pool is no error, the
+// counters then come from the default one.
+void counter_pool_add(ckr_scene *s) {
+  if (s->device < 0 || s->device >= 64) return;
+  CounterPool &c = counter_pool();
+  std::lock_guard<std::mutex> lock(c.mu);
+  if (!c.pool[s->device]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = s->device;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = ~0ull;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return;
+    }
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      (void)cudaGetLastError();
+      cudaMemPoolDestroy(pool);
+      return;
+    }
+    c.pool[s->device] = pool;
+  }
+  ++c.refs[s->device];
+  s->counters = c.pool[s->device];
+}
+
+void counter_pool_drop(ckr_scene *s) {
+  if (!s->counters) return;
+  CounterPool &c = counter_pool();
+  std::lock_guard<std::mutex> lock(c.mu);
+  if (--c.refs[s->device] == 0) {
+    cudaMemPoolDestroy(c.pool[s->device]);  // counters still in use keep their memory until freed
+    c.pool[s->device] = nullptr;
+  }
+  s->counters = nullptr;
+}
+
 // Launches the traversal of rays[0, n).  `next` is a zeroed-per-launch ray counter
 // owned by the caller (one per concurrently used stream), or null to allocate one
-// in stream order for this call.
+// in stream order for this call.  Few rays (up to 32 for each resident warp) are dealt
+// out by the launch itself: no counter, and a grid no larger than they need.
 template <bool ANY>
 int launch_trace(const ckr_scene *s, const ckr_ray *rays, uint32_t n, uint32_t *hit_id, float *hit_t,
                  uint8_t *occluded, cudaStream_t stream, uint32_t *next = nullptr) {
   if (n == 0) return CKR_OK;
-  const int grid = s->trace_grid[ANY ? 1 : 0];
+  const uint32_t full = (uint32_t)s->trace_grid[ANY ? 1 : 0];
+  const uint32_t lanes = dealt_lanes(n, full * (kTPB / 32));
+  const uint32_t grid = lanes ? std::min(full, ceil_div(n, lanes * (kTPB / 32))) : full;
   const size_t smem = s->trace_smem;
+  const TraceFn fn = trace_fn<ANY>(s, lanes != 0);
   // The attribute is per kernel: set it for this scene's stack before each launch.
-  if (smem > 48 * 1024)
-    CKR_CUDA_TRY(cudaFuncSetAttribute(trace_fn<ANY>(s), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) CKR_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // Launches cover at most 2^31 rays so that the counter, which overshoots n by at
   // most one refill per warp, cannot wrap.
-  const bool own = next == nullptr;
-  if (own) CKR_CUDA_TRY(cudaMallocAsync((void **)&next, sizeof(uint32_t), stream));
+  const bool own = !lanes && next == nullptr;
+  if (own) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CKR_CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
+    if (s->counters && capture == cudaStreamCaptureStatusNone)
+      CKR_CUDA_TRY(cudaMallocFromPoolAsync((void **)&next, sizeof(uint32_t), s->counters, stream));
+    else
+      CKR_CUDA_TRY(cudaMallocAsync((void **)&next, sizeof(uint32_t), stream));
+  }
   cudaError_t e = cudaSuccess;
   constexpr uint32_t kChunk = 1u << 31;
   for (uint32_t off = 0; off < n && e == cudaSuccess; off += std::min(n - off, kChunk)) {
     const uint32_t m = std::min(n - off, kChunk);
-    e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
+    if (!lanes) e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) break;
-    trace_fn<ANY>(s)<<<grid, kTPB, smem, stream>>>(
-        view_of(s), reinterpret_cast<const float4 *>(rays + off), m, ANY ? nullptr : hit_id + off,
-        ANY ? nullptr : hit_t + off, ANY ? occluded + off : nullptr, (int)stack_depth_of(s), next);
+    fn<<<grid, kTPB, smem, stream>>>(view_of(s), reinterpret_cast<const float4 *>(rays + off), m,
+                                     ANY ? nullptr : hit_id + off, ANY ? nullptr : hit_t + off,
+                                     ANY ? occluded + off : nullptr, (int)stack_depth_of(s), next, lanes);
     e = cudaGetLastError();
     if (n - off <= kChunk) break;
   }
@@ -209,6 +277,7 @@ extern "C" int ckr_scene_create(const float *tri9, uint32_t ntri, const float *s
   if (cudaMemset(s->status.ptr, 0, sizeof(int)) != cudaSuccess) return fail(CKR_ERR_CUDA);
   LaunchShape l0, l1;
   if (launch_shape<false>(s, l0) != cudaSuccess || launch_shape<true>(s, l1) != cudaSuccess) return fail(CKR_ERR_CUDA);
+  counter_pool_add(s);
   s->trace_grid[0] = l0.grid;
   s->trace_grid[1] = l1.grid;
   s->trace_smem = l0.smem;
@@ -227,6 +296,7 @@ extern "C" int ckr_scene_destroy(ckr_scene *scene) {
   if (scene->user_ready) cudaEventDestroy(scene->user_ready);
   if (scene->h_status) cudaFreeHost(scene->h_status);
   if (scene->render_ws && scene->render_ws_free) scene->render_ws_free(scene->render_ws);
+  counter_pool_drop(scene);
   delete scene;
   return CKR_OK;
 }

@@ -443,12 +443,25 @@ static __device__ __noinline__ uint32_t trace_ray_rt(const SceneView &s, const R
 // were 4 % and 6 % slower on the 1.3M-triangle workload).
 constexpr int kRefill = 8;
 
+// Few rays: when n rays need no more than the 32 lanes of each of the `warps` resident
+// warps, the launch deals them out itself (trace_dealt), this many to each warp (0: more rays than
+// lanes, dynamic fetching).  Up to a quarter of the resident warps (eight per SM) are
+// filled first, then their lanes: the rays of a warp cost more by diverging than a few
+// more warps cost in issue slots (1,013 rays on 1.3M triangles: eight warps per SM 55 us,
+// four 70 us, two 72 us; sixteen as eight).  Dealt out above that, with nothing left to
+// balance the SMs by, 160,000 rays were 5 % slower than with the counter.
+__host__ __device__ __forceinline__ uint32_t dealt_lanes(uint32_t n, uint32_t warps) {
+  if (n > warps * 32u) return 0;
+  const uint32_t l = n / (warps / 4u + 1u) + 1u;
+  return l < 32u ? l : 32u;
+}
+
 // Traversal loop with dynamic ray fetching (after Aila and Laine, "Understanding
 // the Efficiency of Ray Traversal on GPUs", HPG 2009): a lane whose ray is finished
 // takes the next work item from the global counter `next` (one atomicAdd per warp
 // refill, for as many items as the warp has idle lanes) instead of idling until its
 // whole warp is done; each iteration advances every active lane by one trace_step.
-// Taking 32..128 items per atomic into a warp-private range was 4-5 % slower.  The
+// Taking 32..128 items per atomic into a warp-private range was 4-5 % slower. The
 // caller zeroes `next` before the launch and runs every lane of every warp through
 // here (the loop votes over full warps).
 //   fetch(i, r, tbest) -> bool: sets up work item i < n (ray, tmax); false skips it.
@@ -481,12 +494,16 @@ constexpr size_t kSlotLutBytes = 2048;
 
 template <int TPB>
 __device__ __forceinline__ const uint8_t *fill_slot_lut(uint8_t *lut) {
-  for (uint32_t i = threadIdx.x; i < kSlotLutBytes; i += TPB) {
-    const uint32_t o = i >> 8, x = i & 255u;
-    uint32_t y = 0;
-    for (uint32_t b = 0; b < 8; ++b)
-      if (x >> b & 1u) y |= 1u << (b ^ o);
-    lut[i] = (uint8_t)y;
+  // Bit s to bit s ^ oct: for each bit of oct the halves of its size change places.
+  // Four entries to a word; entry by entry and bit by bit the fill took 4 us of every
+  // launch.
+  for (uint32_t i = threadIdx.x; i < kSlotLutBytes / 4; i += TPB) {
+    const uint32_t o = i >> 6, x = (i & 63u) * 4u;
+    uint32_t y = (x * 0x01010101u) + 0x03020100u;  // x, x + 1, x + 2, x + 3
+    if (o & 1u) y = (y & 0x55555555u) << 1 | (y >> 1 & 0x55555555u);
+    if (o & 2u) y = (y & 0x33333333u) << 2 | (y >> 2 & 0x33333333u);
+    if (o & 4u) y = (y & 0x0f0f0f0fu) << 4 | (y >> 4 & 0x0f0f0f0fu);
+    reinterpret_cast<uint32_t *>(lut)[i] = y;
   }
   __syncthreads();
   return lut;
@@ -550,6 +567,25 @@ __device__ __forceinline__ void trace_dynamic(const SceneView &s, uint32_t n, ui
       }
     }
   }
+}
+
+// Few items (dealt_lanes): every warp takes `lanes` of them once, without the counter;
+// the grid has at least n / lanes warps.  Consecutive runs of items go to different
+// blocks: next to each other they would load the SMs unevenly.
+template <bool ANY, class Fetch, class Finish, class Tri>
+__device__ __forceinline__ void trace_dealt(const SceneView &s, uint32_t n, uint32_t lanes, uint2 *stack, int stride,
+                                            int depth, Fetch fetch, Finish finish, Tri tri) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t idx = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * lanes + lane;
+  RayPre r;
+  float tbest;
+  if (lane >= lanes || idx >= n || !fetch(idx, r, tbest)) return;
+  uint32_t best = kMiss;
+  Trav st = trav_start(s, r);
+  bool live = true;
+  if constexpr (Tri::kSpheres) live = trace_spheres_rt<Tri::kSphereLeaving>(s, r, tbest, best, ANY);
+  while (live) live = trace_step<ANY>(s, r, tbest, best, st, stack, stride, depth, tri);
+  finish(idx, best, tbest);
 }
 
 // The same work with one item per thread in a grid-stride loop: faster than
