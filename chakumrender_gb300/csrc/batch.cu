@@ -209,15 +209,14 @@ int enqueue(ckr_batch *b, JobSet &set, bool pack, size_t wave, cudaStream_t stre
       ++n_launch;
       int cur = 0;
       for (uint32_t d = 0; d <= dmax; ++d) {
-        // Work counters of k_extend and k_shadow (P.counts[3], [4]).
-        CKR_CUDA_TRY(cudaMemsetAsync(P.counts + 3, 0, 2 * sizeof(uint32_t), stream));
-        extend_fn<<<g_ext, TPB, smem, stream>>>(sv, P, cur, depth);
-        CKR_CUDA_TRY(cudaMemsetAsync(P.counts + (cur ^ 1), 0, sizeof(uint32_t), stream));
-        CKR_CUDA_TRY(cudaMemsetAsync(P.counts + 2, 0, sizeof(uint32_t), stream));
-        if (nee) k_shade_nee<TPB><<<g_shade, TPB, 0, stream>>>(shv, P, prm, cur, Learn{});
-        else path_fn<<<g_shade, TPB, 0, stream>>>(shv, P, prm, cur, (int)d, nullptr);
-        shadow_fn<<<g_sh, TPB, smem, stream>>>(sv, P, depth, cur, nullptr);
-        n_launch += 3;
+        extend_fn<<<grid_of(g_ext, n, TPB), TPB, smem, stream>>>(sv, P, cur, depth);
+        if (nee) k_shade_nee<TPB><<<grid_of(g_shade, n, TPB), TPB, 0, stream>>>(shv, P, prm, cur, Learn{});
+        else path_fn<<<grid_of(g_shade, n, TPB), TPB, 0, stream>>>(shv, P, prm, cur, (int)d, nullptr);
+        n_launch += 2;
+        if (d < dmax) {  // at the last depth paths only add emission: no shadow rays
+          shadow_fn<<<grid_of(g_sh, (uint64_t)n * b->per_path, TPB), TPB, smem, stream>>>(sv, P, depth, nullptr);
+          ++n_launch;
+        }
         cur ^= 1;
       }
     }

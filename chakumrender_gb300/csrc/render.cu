@@ -153,7 +153,8 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
                           : point_lights + area_lights * prm.n_light + (cfg->shader == CKR_SHADER_DIRECT_MIS ? prm.n_brdf : 0) +
                                 (cfg->shader == CKR_SHADER_DIRECT_MIS || cfg->shader == CKR_SHADER_PATH ? s->env_n : 0);
   if (cfg->shader == CKR_SHADER_DIRECT_CV) per_path = mesh_lights_of(s) * prm.n_light;
-  if (cfg->shader == CKR_SHADER_EXPLICIT) per_path = 0;  // the MISCV direct term traces no shadow rays
+  if (cfg->shader == CKR_SHADER_EXPLICIT || cfg->shader == CKR_SHADER_DIRECT_MISCV)
+    per_path = 0;  // the MISCV direct term traces no shadow rays
   prm.shadow_per_path = std::max(1u, per_path);
   uint64_t total = (uint64_t)prm.npix * prm.spp;
   size_t wave = (size_t)std::min<uint64_t>(total, std::max<uint64_t>(32768, (1ull << 23) / prm.shadow_per_path));
@@ -263,14 +264,10 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
   // One step of the wavefront over queue `cur`: closest hit, [learned selection],
   // shading, shadow rays, [training].  k: the step's index within the wave (or the
   // render, with regeneration) -- it picks the selection buffer, and k = 0 has no
-  // previous one; nee: the step's vertices may draw light samples.
+  // previous one; nee: the step's vertices may draw light samples; n: paths at most.
   int cur = 0;
-  auto step = [&](uint64_t k, bool nee) -> int {
-    // Work counters of k_extend and k_shadow (P.counts[3], [4]).
-    CKR_CUDA_TRY(cudaMemsetAsync(P.counts + 3, 0, 2 * sizeof(uint32_t), stream));
-    extend_fn<<<g_ext, kRTPB, smem, stream>>>(sv, P, cur, depth);
-    CKR_CUDA_TRY(cudaMemsetAsync(P.counts + (cur ^ 1), 0, sizeof(uint32_t), stream));
-    CKR_CUDA_TRY(cudaMemsetAsync(P.counts + 2, 0, sizeof(uint32_t), stream));
+  auto step = [&](uint64_t k, bool nee, uint32_t n) -> int {
+    extend_fn<<<grid_of(g_ext, n, kRTPB), kRTPB, smem, stream>>>(sv, P, cur, depth);
     Learn lr{};
     if (prop) lr.sel_prev = k ? prop->sel[(k - 1) & 1].ptr : nullptr;
     // Overlapped training: this step uses record buffer and weight copy b, which the
@@ -313,8 +310,11 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
       }
     }
     const int d = (int)std::min<uint64_t>(k, prm.max_depth);
-    shade.launch(g_shade, cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, stream, shv, P, prm, cur, d, ltc, sv, depth, lr);
-    shadow_fn<<<g_sh, kRTPB, smem, stream>>>(sv, P, depth, cur, train && nee ? rec : nullptr);
+    shade.launch(grid_of(g_shade, n, kRTPB), cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, stream, shv, P, prm, cur, d,
+                 ltc, sv, depth, lr);
+    if (nee && per_path)  // else the step has no shadow rays
+      shadow_fn<<<grid_of(g_sh, (uint64_t)n * per_path, kRTPB), kRTPB, smem, stream>>>(sv, P, depth,
+                                                                                      train ? rec : nullptr);
     if (train && nee) {
       // Adam steps on this step's light samples (visibility applied above),
       // minibatch by minibatch; steps past the records actually written are no-ops.
@@ -366,7 +366,7 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
     // max_depth + 1: a bound on the steps in case the read-back never sees zero.
     const uint64_t max_steps = ceil_div(total, wave) * (uint64_t)(prm.max_depth + 1) + prm.max_depth + 2;
     for (uint64_t k = 0; k < max_steps; ++k) {
-      int st = step(k, true);
+      int st = step(k, true, (uint32_t)wave);
       if (st != CKR_OK) return st;
       CKR_CUDA_TRY(cudaMemcpyAsync(W.h_count + (k & 1), P.counts + cur, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                    stream));
@@ -382,9 +382,9 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
       k_camera<kRTPB><<<std::min<int>(g_ext, ceil_div(n, kRTPB)), kRTPB, 0, stream>>>(c, P, prm, base, n);
       cur = 0;
       for (uint32_t d = 0; d <= prm.max_depth; ++d) {
-        // The vertices at the last depth only add emission: no light sample, so
-        // neither a light distribution nor training records there.
-        int st = step(d, d < prm.max_depth);
+        // The vertices at the last depth of a path only add emission: no light sample, so
+        // neither a light distribution nor training records nor shadow rays there.
+        int st = step(d, d < prm.max_depth, n);
         if (st != CKR_OK) return st;
         if (!path) break;
       }
@@ -577,7 +577,9 @@ extern "C" int ckr_render_noalloc(ckr_scene *s, const ckr_camera *cam, const ckr
                                 (cfg->shader == CKR_SHADER_DIRECT_MIS ? prm.n_brdf : 0) +
                                 (cfg->shader == CKR_SHADER_DIRECT_MIS || cfg->shader == CKR_SHADER_PATH ? s->env_n : 0);
   if (cfg->shader == CKR_SHADER_DIRECT_CV) per_path = (uint64_t)mesh_lights_of(s) * prm.n_light;
-  if (cfg->shader == CKR_SHADER_EXPLICIT) per_path = 0;  // the MISCV direct term traces no shadow rays
+  if (cfg->shader == CKR_SHADER_EXPLICIT) per_path = 0;
+  // The MISCV direct term traces no shadow rays.
+  const bool shadows = cfg->shader != CKR_SHADER_EXPLICIT && cfg->shader != CKR_SHADER_DIRECT_MISCV && per_path;
   if (per_path > kNoAllocShadow) return CKR_ERR_TOO_LARGE;
   prm.shadow_per_path = (uint32_t)std::max<uint64_t>(1, per_path);
   uint64_t total = (uint64_t)prm.npix * prm.spp;
@@ -643,14 +645,11 @@ extern "C" int ckr_render_noalloc(ckr_scene *s, const ckr_camera *cam, const ckr
     k_camera<kRTPB><<<std::min<int>(g_ext, ceil_div(n, kRTPB)), kRTPB, 0, stream>>>(c, P, prm, base, n);
     int cur = 0;
     for (uint32_t d = 0; d <= prm.max_depth; ++d) {
-      // Work counters of k_extend and k_shadow (P.counts[3], [4]).
-      CKR_CUDA_TRY(cudaMemsetAsync(P.counts + 3, 0, 2 * sizeof(uint32_t), stream));
-      extend_fn<<<g_ext, kRTPB, smem, stream>>>(sv, P, cur, depth);
-      CKR_CUDA_TRY(cudaMemsetAsync(P.counts + (cur ^ 1), 0, sizeof(uint32_t), stream));
-      CKR_CUDA_TRY(cudaMemsetAsync(P.counts + 2, 0, sizeof(uint32_t), stream));
-      shade.launch(g_shade, cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, stream, shv, P, prm, cur, (int)d, ltc, sv,
-                   depth, Learn{});
-      shadow_fn<<<g_sh, kRTPB, smem, stream>>>(sv, P, depth, cur, nullptr);
+      extend_fn<<<grid_of(g_ext, n, kRTPB), kRTPB, smem, stream>>>(sv, P, cur, depth);
+      shade.launch(grid_of(g_shade, n, kRTPB), cfg->shader == CKR_SHADER_EXPLICIT ? smem : 0, stream, shv, P, prm, cur,
+                   (int)d, ltc, sv, depth, Learn{});
+      if (d < prm.max_depth && shadows)  // else the step has no shadow rays
+        shadow_fn<<<grid_of(g_sh, n * per_path, kRTPB), kRTPB, smem, stream>>>(sv, P, depth, nullptr);
       cur ^= 1;
       if (!path) break;
     }

@@ -68,8 +68,11 @@ struct Paths {
   uint32_t *sh_px;
   uint32_t *prev_row;  // learned selection: the path's row in the previous bounce's probabilities
   uint32_t *sh_rec;    // training: per shadow ray, its training record (kNoRec: none)
-  uint32_t *counts;  // [0] q[0] length, [1] q[1] length, [2] shadow count, [3] [4] work counters of
-                     // k_extend and k_shadow (zeroed before each k_extend)
+  // [0] q[0] length, [1] q[1] length, [2] shadow count, [3] [4] work counters of k_extend
+  // and k_shadow, [5] next camera path to start.  A step's kernels clear them for each
+  // other, in launch order: k_camera and the shading kernel [3], k_extend what the shading
+  // kernel and k_shadow fill (a memset node costs 3 us of a captured step, a memset 1 us).
+  uint32_t *counts;
   unsigned long long *stats;  // cumulative closest-hit rays, shadow rays
   double *accum;     // 3 per output pixel
   uint32_t sh_cap;   // shadow-queue capacity (rays)
@@ -233,6 +236,7 @@ __global__ void __launch_bounds__(TPB) k_camera(Cam cam0, Paths P, Params prm, u
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     P.counts[0] = wave_n;
+    P.counts[3] = 0;
     P.counts[5] = (uint32_t)(wave_base + wave_n);
   }
 }
@@ -274,6 +278,12 @@ template <int TPB, Walk WALK>
 __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_extend(SceneView s, Paths P, int cur, int depth) {
   extern __shared__ uint2 smem_trav[];
   const uint32_t *q = cur ? P.q1 : P.q0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    P.counts[cur ^ 1] = 0;
+    P.counts[2] = 0;
+    P.counts[4] = 0;
+    atomicAdd(&P.stats[0], (unsigned long long)P.counts[cur]);  // ray statistics: this step's closest-hit rays
+  }
   auto fetch = [&](uint32_t i, RayPre &r, float &tmax) {
     const uint32_t slot = q[i];
     const float4 a = P.ray_o[slot], b = P.ray_d[slot];
@@ -304,14 +314,11 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_extend(SceneView s, 
 // pixel; occluded ones zero their training record's weight.  Dynamic
 // fetching takes its work from the counter P.counts[4] (zeroed before the launch).
 template <int TPB, Walk WALK>
-__global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, Paths P, int depth, int cur, float4 *rec) {
+__global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, Paths P, int depth, float4 *rec) {
   extern __shared__ uint2 smem_trav[];
   const uint32_t n = min(P.counts[2], P.sh_cap);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    // Ray statistics: closest-hit rays of this bounce and its shadow rays.
-    atomicAdd(&P.stats[0], (unsigned long long)P.counts[cur]);
-    atomicAdd(&P.stats[1], (unsigned long long)n);
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    atomicAdd(&P.stats[1], (unsigned long long)n);  // ray statistics: this step's shadow rays
   auto fetch = [&](uint32_t i, RayPre &r, float &tmax) {
     const float4 a = P.sh_o[i], b = P.sh_d[i];
     r = make_ray(a, b);
@@ -341,7 +348,7 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, 
 }
 
 using ExtendFn = void (*)(SceneView, Paths, int, int);
-using ShadowFn = void (*)(SceneView, Paths, int, int, float4 *);
+using ShadowFn = void (*)(SceneView, Paths, int, float4 *);
 inline Walk walk_of(const ckr_scene *s) {
   return s->max_depth < kDynamicDepth ? kWalkStatic : s->nsph ? kWalkDyn : kWalkDynNoSpheres;
 }
@@ -518,6 +525,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
   const uint32_t n = P.counts[cur];
   const uint32_t *q = cur ? P.q1 : P.q0;
   uint32_t *qn = cur ? P.q0 : P.q1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) P.counts[3] = 0;
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (TPB / 32);
   const uint32_t warp_id = blockIdx.x * (TPB / 32) + (threadIdx.x >> 5);
@@ -828,6 +836,7 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
   const uint32_t n = P.counts[cur];
   const uint32_t *q = cur ? P.q1 : P.q0;
   uint32_t *qn = cur ? P.q0 : P.q1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) P.counts[3] = 0;
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (TPB / 32);
   const uint32_t warp_id = blockIdx.x * (TPB / 32) + (threadIdx.x >> 5);
@@ -1005,6 +1014,10 @@ __global__ void k_resolve(const double *accum, float *rgb, uint32_t n3, double i
     rgb[i] = (float)(accum[i] * inv_spp);
 }
 
+
+// Blocks for up to n items: the persistent grid g, or fewer where n fill fewer (an
+// empty block of a full grid costs about as much as one that works).
+inline unsigned grid_of(int g, uint64_t n, int tpb) { return (unsigned)std::min<uint64_t>(g, std::max<uint64_t>(1, (n + tpb - 1) / tpb)); }
 
 int grid_for(const void *fn, size_t smem, int tpb) {
   int dev = 0, sms = 0, per = 0;
