@@ -15,9 +15,9 @@
 // gradient G (rows b):  dW^T = X^T G  (M = input features padded to 128,
 // N = 64, K = the 128 rows of the tile), accumulated in TMEM across all tiles a
 // CTA processes, and dX = G W  (M = 128 rows, N = 64, K = 64) for the layer
-// below.  The transposed operands X^T and G^T are written to shared memory by
-// the epilogues.  Row 64 of X^T is all ones, so row 64 of dW^T is the bias
-// gradient (the first layer's bias is the weight of its constant feature).
+// below.  X^T and G^T are X and G read as MN-major operands.  Column 64 of X is all
+// ones, so row 64 of dW^T is the bias gradient (the first layer's bias is the weight of
+// its constant feature).
 //
 // Bounds: every mbarrier wait gives up after kWaitTries polls, records
 // CKR_ERR_ITERATION_LIMIT, waits once more (bounded) for the MMAs in flight,
@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "ckr_internal.h"
@@ -40,7 +41,7 @@ namespace mlp {
 namespace {
 
 constexpr uint32_t kWaitTries = 1u << 22;
-constexpr uint32_t kIdesc = tc::idesc_bf16(128, 64);
+constexpr uint32_t kIdesc = tc::idesc_bf16(128, 64), kIdescT = tc::idesc_bf16(128, 64, true);
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -59,10 +60,6 @@ __device__ __forceinline__ void ld8(const uint8_t *op, uint32_t r, uint32_t k0, 
   v[0] = bf16_lo(q.x); v[1] = bf16_hi(q.x); v[2] = bf16_lo(q.y); v[3] = bf16_hi(q.y);
   v[4] = bf16_lo(q.z); v[5] = bf16_hi(q.z); v[6] = bf16_lo(q.w); v[7] = bf16_hi(q.w);
 }
-__device__ __forceinline__ void st1(uint8_t *op, uint32_t r, uint32_t k, uint32_t K, float v) {
-  *reinterpret_cast<__nv_bfloat16 *>(op + tc::kmaj(r, k, K)) = __float2bfloat16_rn(v);
-}
-
 // Rows to process: n_max, or what the device count leaves after n_off.
 __device__ __forceinline__ uint32_t rows(uint32_t n_max, const uint32_t *n_dev, uint32_t n_off) {
   if (!n_dev) return n_max;
@@ -78,7 +75,9 @@ struct Params {
   uint32_t stall_tries;
 };
 
-// Row features into the first-layer operand (K = 96).
+// Row features into the first-layer operand (K = 96): the 8-feature groups of PART 0 (the
+// first two coordinates), 1 (the third and the rest) or 2 (all).
+template <int PART = 2>
 __device__ __forceinline__ void write_features(uint8_t *x0, uint32_t t, float4 r0, float4 r1, float4 r2,
                                                const Params &p) {
   float f[kIn];
@@ -88,7 +87,7 @@ __device__ __forceinline__ void write_features(uint8_t *x0, uint32_t t, float4 r
   // (about 1e-6 at the base) roughly doubles per octave, a few 1e-3 after eleven,
   // at the level of BF16's rounding of the features.
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
+  for (int c = PART == 1 ? 2 : 0; c < (PART == 0 ? 2 : 3); ++c) {
     float sn, cs;
     __sincosf(3.14159265358979f * pc[c], &sn, &cs);  // |argument| <= pi inside the scene box
 #pragma unroll
@@ -107,7 +106,7 @@ __device__ __forceinline__ void write_features(uint8_t *x0, uint32_t t, float4 r
 #pragma unroll
   for (int j = 80; j < (int)kIn; ++j) f[j] = 0.f;
 #pragma unroll
-  for (int q = 0; q < (int)kIn / 8; ++q) st8(x0, t, 8 * q, kIn, f + 8 * q);
+  for (int q = PART == 1 ? 6 : 0; q < (PART == 0 ? 6 : (int)kIn / 8); ++q) st8(x0, t, 8 * q, kIn, f + 8 * q);
 }
 
 // Two FP32 values to a BF16 pair with ReLU (lower half = first value).
@@ -120,9 +119,9 @@ __device__ __forceinline__ uint32_t pack_relu_bf16(float lo, float hi) {
 // Accumulator row t (64 columns, bias included by the MMA) through ReLU into row t
 // of a hidden-layer operand (K = 80): columns 0..63, then the constant 1 at 64 and
 // zeros to 79.
-__device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t *dst, uint32_t t) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
+__device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t *dst, uint32_t t, int h0 = 0, int h1 = 2) {
+#pragma unroll 2
+  for (int h = h0; h < h1; ++h) {
     float v[32];
     tc::tmem_ld32(taddr + 32 * h, v);
 #pragma unroll
@@ -133,6 +132,7 @@ __device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t *dst, uint
                      pack_relu_bf16(x[6], x[7]));
     }
   }
+  if (h1 < 2) return;  // halves [h0, h1) of the columns; the constants go with the second
   *reinterpret_cast<uint4 *>(dst + tc::kmaj(t, 64, kHidK)) = make_uint4(0x3F80u, 0u, 0u, 0u);  // BF16 1.0
   *reinterpret_cast<uint4 *>(dst + tc::kmaj(t, 72, kHidK)) = make_uint4(0u, 0u, 0u, 0u);
 }
@@ -172,6 +172,12 @@ __device__ __forceinline__ float softmax_exp(uint32_t taddr, uint32_t C, float *
 __device__ __forceinline__ void issue(uint32_t d, uint32_t a, uint32_t b, uint32_t K, uint32_t accumulate_first) {
   for (uint32_t s = 0; s < K / 16; ++s)
     tc::mma_bf16(d, tc::sdesc(a, K, s), tc::sdesc(b, K, s), kIdesc, (s > 0 || accumulate_first) ? 1u : 0u);
+}
+
+// D (+)= X^T G over the 128 rows of a tile: X stored [128 x C], G [128 x 64].
+__device__ __forceinline__ void issue_t(uint32_t d, uint32_t x, uint32_t C, uint32_t g, uint32_t accumulate_first) {
+  for (uint32_t s = 0; s < 8; ++s)
+    tc::mma_bf16(d, tc::sdesc_t(x, C, s), tc::sdesc_t(g, 64, s), kIdescT, (s > 0 || accumulate_first) ? 1u : 0u);
 }
 
 // Barrier of one 128-thread group (named barrier 1 + g; 0 is __syncthreads).
@@ -399,17 +405,20 @@ __global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(const float4 *__rest
 }
 
 // ---- training -------------------------------------------------------------------
-constexpr uint32_t kTrainTPB = 128;
+// Two threads per row: thread (t, hf) of a tile computes half hf of row t's features,
+// epilogues and transposes (columns 32 hf .. +31), the halves in warps w and w + 4, which
+// read the same TMEM lanes.  The softmax's sum runs over all 64 columns in both, in the
+// same order.
+constexpr uint32_t kTrainTPB = 256;
 
 struct SmemTrain {
   uint8_t w[kImgBytes];
   uint8_t x0[128 * kIn * 2];
   uint8_t h[3][128 * kHidK * 2];  // H1, H2, H3 with the constant-1 column (K = 80)
+  // X^T reads up to 768 bytes past x0 and h (sdesc_t): into what follows here.
   uint8_t g[128 * 64 * 2];        // G [128 rows x K 64]
-  uint8_t gt[64 * 128 * 2];       // G^T [64 x K 128]
-  uint8_t ht[128 * 128 * 2];      // X^T [128 (features, padded) x K 128]
-  float loss[kTrainTPB / 32];
-  uint64_t mbar;
+  float loss[4];
+  uint64_t mbar, mbar_w;
   uint32_t tmem;
   int abort;
 };
@@ -418,6 +427,34 @@ constexpr uint32_t kColD = 0;
 // TMEM column of the dW^T accumulator of layer l = 0..3 (dW1..dW4).
 __device__ __forceinline__ uint32_t col_w(int l) { return 256u - 64u * (uint32_t)l; }
 
+// As sync_for_mma and wait_mma, for the whole block.
+__device__ __forceinline__ void block_sync_for_mma() {
+  tc::fence_proxy_async();
+  tc::fence_before_sync();
+  __syncthreads();
+}
+__device__ __forceinline__ bool block_wait_mma(uint32_t mbar, uint32_t &phase, int *abort, int *err) {
+  if (!tc::mbar_wait(mbar, phase, kWaitTries)) {
+    *abort = 1;
+    atomicExch(err, CKR_ERR_ITERATION_LIMIT);
+  }
+  __syncthreads();
+  if (*abort) {
+    tc::mbar_wait(mbar, phase, kWaitTries);  // let the MMAs in flight land before TMEM is freed
+    return false;
+  }
+  phase ^= 1u;
+  tc::fence_after_sync();
+  return true;
+}
+
+// Latency bound: a CTA's tile is a chain of eight MMA groups with an epilogue between each
+// two.  So: two threads a row; the weight images by one bulk copy beside the features; X^T
+// and G^T read in place as MN-major operands (copied by the threads, 2 bytes a store and
+// four-way bank conflicts, they were 5 of the kernel's 20 us); and the batch's weight sum
+// (k_mlp_wsum, the launch before), which only the loss needs, overlapping the forward pass
+// (programmatic dependent launch).  A step of 4,096 records: 39.4 -> 21.8 us, this kernel
+// 24.0 -> 14.6 us.
 __global__ void __launch_bounds__(kTrainTPB) k_mlp_train(const float4 *__restrict__ rec, uint32_t n_max,
                                                          const uint32_t *n_dev, uint32_t n_off,
                                                          const uint8_t *__restrict__ img, const float *scalars,
@@ -425,29 +462,26 @@ __global__ void __launch_bounds__(kTrainTPB) k_mlp_train(const float4 *__restric
                                                          int *err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   SmemTrain &S = *reinterpret_cast<SmemTrain *>(smem_raw);
-  const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  for (uint32_t i = t; i < kImgBytes / 16; i += kTrainTPB)
-    reinterpret_cast<uint4 *>(S.w)[i] = reinterpret_cast<const uint4 *>(img)[i];
-  for (uint32_t i = t; i < sizeof(S.ht) / 16; i += kTrainTPB)
-    reinterpret_cast<uint4 *>(S.ht)[i] = make_uint4(0, 0, 0, 0);
-  const uint32_t mbar = tc::smem_u32(&S.mbar);
-  if (t == 0) {
+  const uint32_t t = threadIdx.x & 127u, hf = threadIdx.x >> 7, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  tc::launch_dependents();
+  const uint32_t mbar = tc::smem_u32(&S.mbar), mbar_w = tc::smem_u32(&S.mbar_w);
+  if (threadIdx.x == 0) {
     tc::mbar_init(mbar, 1);
+    tc::mbar_init(mbar_w, 1);
     S.abort = 0;
+    tc::bulk_load(tc::smem_u32(S.w), img, kImgBytes, mbar_w);
   }
   if (warp == 0) tc::tmem_alloc(&S.tmem, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = S.tmem, lane_addr = tmem + ((warp * 32u) << 16);
+  const uint32_t tmem = S.tmem, lane_addr = tmem + (((warp & 3u) * 32u) << 16);
   const uint32_t n = rows(n_max, n_dev, n_off);
-  const float wsum = scalars[0];
-  const uint32_t w_addr = tc::smem_u32(S.w), x0_addr = tc::smem_u32(S.x0), g_addr = tc::smem_u32(S.g),
-                 gt_addr = tc::smem_u32(S.gt), ht_addr = tc::smem_u32(S.ht);
+  const uint32_t w_addr = tc::smem_u32(S.w), x0_addr = tc::smem_u32(S.x0), g_addr = tc::smem_u32(S.g);
   const uint32_t h0_addr = tc::smem_u32(S.h[0]);  // H1, H2, H3 are 20 KB apart
   uint32_t phase = 0, tiles = 0;
-  float loss = 0.f;
-  bool ok = wsum > 0.f;
+  float loss = 0.f, wsum = 0.f;
+  bool ok = true;
   for (uint32_t tile = blockIdx.x; ok && tile * 128u < n; tile += gridDim.x, ++tiles) {
     const uint32_t row = tile * 128u + t;
     float4 r0 = make_float4(0, 0, 0, 0), r1 = r0, r2 = r0;
@@ -456,24 +490,38 @@ __global__ void __launch_bounds__(kTrainTPB) k_mlp_train(const float4 *__restric
       r1 = rec[3 * (size_t)row + 1];
       r2 = rec[3 * (size_t)row + 2];
     }
-    const float a = (row < n && r1.w > 0.f) ? r1.w / wsum : 0.f;
     const uint32_t k = min(__float_as_uint(r2.w), 63u);
     const uint32_t acc = tiles ? 1u : 0u;
     // ---- forward ----
-    write_features(S.x0, t, r0, r1, r2, p);
+    if (hf == 0) write_features<0>(S.x0, t, r0, r1, r2, p);
+    else write_features<1>(S.x0, t, r0, r1, r2, p);
+    if (tiles == 0 && threadIdx.x == 0 && !tc::mbar_wait(mbar_w, 0, kWaitTries)) {
+      S.abort = 1;
+      atomicExch(err, CKR_ERR_ITERATION_LIMIT);
+    }
     for (int l = 0; l < 4 && ok; ++l) {
-      sync_for_mma(0);
-      if (t == 0) {
+      block_sync_for_mma();
+      if (S.abort) {
+        ok = false;  // the weights never arrived
+        break;
+      }
+      if (threadIdx.x == 0) {
         tc::fence_after_sync();
         if (l == 0) issue(tmem + kColD, x0_addr, w_addr + kImgW1, kIn, 0);
         else issue(tmem + kColD, h0_addr + 20480u * (l - 1), w_addr + kImgW2 + 10240u * (l - 1), kHidK, 0);
         tc::mma_commit(mbar);
       }
-      ok = wait_mma(0, mbar, phase, &S.abort, err);
-      if (ok && l < 3) epilogue_relu(lane_addr + kColD, S.h[l], t);
+      ok = block_wait_mma(mbar, phase, &S.abort, err);
+      if (ok && l < 3) epilogue_relu(lane_addr + kColD, S.h[l], t, hf, hf + 1);
     }
     if (!ok) break;
     // ---- loss gradient at the logits: a (softmax - onehot(k)) ----
+    if (tiles == 0) {
+      tc::wait_dependencies();
+      wsum = __ldcg(scalars);
+      if (!(wsum > 0.f)) break;  // nothing to learn: no partial sums
+    }
+    const float a = (row < n && r1.w > 0.f) ? r1.w / wsum : 0.f;
     {
       float pr[64];
       const float inv = 1.0f / softmax_exp(lane_addr + kColD, p.nclusters, pr);
@@ -483,101 +531,84 @@ __global__ void __launch_bounds__(kTrainTPB) k_mlp_train(const float4 *__restric
         pr[j] *= inv;
         pk = (uint32_t)j == k ? pr[j] : pk;
       }
-      if (a > 0.f) loss -= a * __logf(fmaxf(pk, 1e-30f));
+      if (a > 0.f && hf == 0) loss -= a * __logf(fmaxf(pk, 1e-30f));
 #pragma unroll
       for (int j = 0; j < 64; ++j) pr[j] = (uint32_t)j < p.nclusters ? a * (pr[j] - ((uint32_t)j == k ? 1.f : 0.f)) : 0.f;
+      if (hf == 0) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) st8(S.g, t, 8 * q, 64, pr + 8 * q);
+        for (int q = 0; q < 4; ++q) st8(S.g, t, 8 * q, 64, pr + 8 * q);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 64; ++j) st1(S.gt, j, t, 128, pr[j]);
+        for (int q = 4; q < 8; ++q) st8(S.g, t, 8 * q, 64, pr + 8 * q);
+      }
     }
+    const uint32_t j0 = 32u * hf;
     // ---- backward, layers 4, 3, 2 (input H3, H2, H1) ----
     for (int l = 2; l >= 0 && ok; --l) {
-      // X^T of the layer's input with the ones row (64) for the bias.
-      {
-        float v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          ld8(S.h[l], t, 8 * q, kHidK, v);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) st1(S.ht, 8 * q + j, t, 128, v[j]);
-        }
-        st1(S.ht, 64, t, 128, 1.0f);
-      }
-      sync_for_mma(0);
-      if (t == 0) {
+      block_sync_for_mma();
+      if (threadIdx.x == 0) {
         tc::fence_after_sync();
-        issue(tmem + col_w(l + 1), ht_addr, gt_addr, 128, acc);            // dW^T += X^T G
-        issue(tmem + kColD, g_addr, w_addr + kImgW2t + 8192u * l, 64, 0);  // dX = G W
+        issue_t(tmem + col_w(l + 1), h0_addr + 20480u * l, kHidK, g_addr, acc);  // dW^T += X^T G
+        issue(tmem + kColD, g_addr, w_addr + kImgW2t + 8192u * l, 64, 0);        // dX = G W
         tc::mma_commit(mbar);
       }
-      if (!(ok = wait_mma(0, mbar, phase, &S.abort, err))) break;
+      // The layer's ReLU mask, while the MMAs run.
+      float hv[32], d[32];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ld8(S.h[l], t, j0 + 8 * q, kHidK, hv + 8 * q);
+      if (!(ok = block_wait_mma(mbar, phase, &S.abort, err))) break;
       // G of the layer below: dX masked by its ReLU.
-      float d[64], hv[64];
-      tc::tmem_ld32(lane_addr + kColD, d);
-      tc::tmem_ld32(lane_addr + kColD + 32, d + 32);
+      tc::tmem_ld32(lane_addr + kColD + j0, d);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) ld8(S.h[l], t, 8 * q, kHidK, hv + 8 * q);
+      for (int j = 0; j < 32; ++j) d[j] = hv[j] > 0.f ? d[j] : 0.f;
 #pragma unroll
-      for (int j = 0; j < 64; ++j) d[j] = hv[j] > 0.f ? d[j] : 0.f;
-      if (l > 0) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) st8(S.g, t, 8 * q, 64, d + 8 * q);
-      }
-#pragma unroll
-      for (int j = 0; j < 64; ++j) st1(S.gt, j, t, 128, d[j]);
+      for (int q = 0; q < 4; ++q) st8(S.g, t, j0 + 8 * q, 64, d + 8 * q);
     }
     if (!ok) break;
     // ---- layer 1: dW1^T += X0^T G1 ----
-    {
-      float v[8];
-#pragma unroll
-      for (int q = 0; q < (int)kIn / 8; ++q) {
-        ld8(S.x0, t, 8 * q, kIn, v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) st1(S.ht, 8 * q + j, t, 128, v[j]);
-      }
-    }
-    sync_for_mma(0);
-    if (t == 0) {
+    block_sync_for_mma();
+    if (threadIdx.x == 0) {
       tc::fence_after_sync();
-      issue(tmem + col_w(0), ht_addr, gt_addr, 128, acc);
+      issue_t(tmem + col_w(0), x0_addr, kIn, g_addr, acc);
       tc::mma_commit(mbar);
     }
-    if (!(ok = wait_mma(0, mbar, phase, &S.abort, err))) break;
+    if (!(ok = block_wait_mma(mbar, phase, &S.abort, err))) break;
     tc::fence_before_sync();
     __syncthreads();
   }
+  // A block without a tile has not waited for its weights, nor for the launch before.
+  if (tiles == 0) {
+    tc::mbar_wait(mbar_w, 0, kWaitTries);
+    tc::wait_dependencies();
+  }
   // ---- per-CTA partial sums ----
   for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-  if (lane == 0) S.loss[warp] = loss;
+  if (lane == 0 && hf == 0) S.loss[warp] = loss;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   float *my = part + (size_t)blockIdx.x * kNParams;
   const bool have = ok && tiles > 0;
-  if (t == 0) loss_part[blockIdx.x] = have ? S.loss[0] + S.loss[1] + S.loss[2] + S.loss[3] : 0.f;
-  // Row i = 32 * warp + lane of each dW^T accumulator: weights of input i, or
-  // (row 64 of layers 2-4) the bias.
-  const uint32_t i = warp * 32u + lane;
+  if (threadIdx.x == 0) loss_part[blockIdx.x] = have ? S.loss[0] + S.loss[1] + S.loss[2] + S.loss[3] : 0.f;
+  // Row t (a TMEM lane) of each dW^T accumulator: weights of input t, or (row 64 of
+  // layers 2-4) the bias.
   for (int l = 0; l < 4; ++l) {
     const uint32_t fan = l == 0 ? kIn : 64;
-    float v[64];
+    float v[32];
     if (have) {
-      tc::tmem_ld32(lane_addr + col_w(l), v);
-      tc::tmem_ld32(lane_addr + col_w(l) + 32, v + 32);
+      tc::tmem_ld32(lane_addr + col_w(l) + 32u * hf, v);
     } else {
 #pragma unroll
-      for (int j = 0; j < 64; ++j) v[j] = 0.f;
+      for (int j = 0; j < 32; ++j) v[j] = 0.f;
     }
     const uint32_t offW = l == 0 ? kOffW1 : l == 1 ? kOffW2 : l == 2 ? kOffW3 : kOffW4;
     const uint32_t offB = l == 1 ? kOffB2 : l == 2 ? kOffB3 : kOffB4;
-    if (i < fan) {
+    if (t < fan) {
 #pragma unroll
-      for (int o = 0; o < 64; ++o) my[offW + o * fan + i] = v[o];
-    } else if (l > 0 && i == 64) {
+      for (int o = 0; o < 32; ++o) my[offW + (32u * hf + o) * fan + t] = v[o];
+    } else if (l > 0 && t == 64) {
 #pragma unroll
-      for (int o = 0; o < 64; ++o) my[offB + o] = v[o];
+      for (int o = 0; o < 32; ++o) my[offB + 32u * hf + o] = v[o];
     }
   }
   tc::fence_before_sync();
@@ -589,6 +620,7 @@ __global__ void __launch_bounds__(kTrainTPB) k_mlp_train(const float4 *__restric
 __global__ void k_mlp_wsum(const float4 *__restrict__ rec, uint32_t n_max, const uint32_t *n_dev, uint32_t n_off,
                            float *scalars) {
   __shared__ float red[32];
+  tc::launch_dependents();  // the training kernel's forward pass does not need the sum
   const uint32_t n = rows(n_max, n_dev, n_off);
   float s = 0.f;
   for (uint32_t r = threadIdx.x; r < n; r += blockDim.x) {
@@ -632,8 +664,10 @@ __global__ void k_mlp_adam(float *params, float *m, float *v, const float *part,
                            const float *loss_part, float *scalars, uint8_t *img, int update, float lr, float b1,
                            float b2, float eps, float c1, float c2) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (update) tc::wait_dependencies();
   if (update && blockIdx.x == 0 && threadIdx.x == 0 && scalars[0] > 0.f) {
     float l = 0.f;
+#pragma unroll 16
     for (uint32_t c = 0; c < grid; ++c) l += loss_part[c];
     scalars[1] = l;
   }
@@ -641,6 +675,7 @@ __global__ void k_mlp_adam(float *params, float *m, float *v, const float *part,
   float w = params[j];
   if (update && scalars[0] > 0.f) {
     float g = 0.f;
+#pragma unroll 16
     for (uint32_t c = 0; c < grid; ++c) g += part[(size_t)c * kNParams + j];
     float mj = b1 * m[j] + (1.f - b1) * g, vj = b2 * v[j] + (1.f - b2) * g * g;
     m[j] = mj;
@@ -773,12 +808,39 @@ int infer_paths(const Net &net, const PathRows &rows, uint32_t n_max, const uint
   return launch_infer<true>(net, nullptr, rows, n_max, n_dev, nullptr, cdf16, delta, stream, img);
 }
 
+namespace {
+template <class T>
+struct Same {
+  using type = T;
+};
+// A launch that may start before the stream's previous kernel has ended; the kernel waits
+// for it where it needs it (tc::wait_dependencies).
+template <class... A>
+cudaError_t launch_early(void (*fn)(A...), uint32_t grid, uint32_t tpb, size_t smem, cudaStream_t stream,
+                         typename Same<A>::type... a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(tpb);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, a...);
+}
+}  // namespace
+
 int gradients(Net &net, const float4 *rec, uint32_t n_max, const uint32_t *n_dev, uint32_t n_off,
               cudaStream_t stream) {
+  // One block per 128-record tile: with the grid fixed at one block per SM, the blocks
+  // without a tile wrote zero partial sums (74 KB each) for k_mlp_adam to add.
+  net.used = std::max<uint32_t>(1, std::min(net.grid, (uint32_t)ceil_div(n_max, 128)));
   k_mlp_wsum<<<1, 1024, 0, stream>>>(rec, n_max, n_dev, n_off, net.scalars);
-  k_mlp_train<<<net.grid, kTrainTPB, sizeof(SmemTrain), stream>>>(rec, n_max, n_dev, n_off, net.img, net.scalars,
-                                                            params_of(net), net.part, net.loss_part, net.err);
   CKR_CUDA_TRY(cudaGetLastError());
+  CKR_CUDA_TRY(launch_early(k_mlp_train, net.used, kTrainTPB, sizeof(SmemTrain), stream, rec, n_max, n_dev, n_off,
+                            net.img, net.scalars, params_of(net), net.part, net.loss_part, net.err));
   return CKR_OK;
 }
 
@@ -789,10 +851,9 @@ int train_step(Net &net, const float4 *rec, uint32_t n_max, const uint32_t *n_de
   if (st != CKR_OK) return st;
   net.step += 1;
   const float c1 = 1.0f - std::pow(net.beta1, (float)net.step), c2 = 1.0f - std::pow(net.beta2, (float)net.step);
-  k_mlp_adam<<<ceil_div(kNParams, 256), 256, 0, stream>>>(net.params, net.m, net.v, net.part, net.grid,
-                                                           net.loss_part, net.scalars, net.img, 1, net.lr, net.beta1,
-                                                           net.beta2, net.eps, c1, c2);
-  CKR_CUDA_TRY(cudaGetLastError());
+  CKR_CUDA_TRY(launch_early(k_mlp_adam, ceil_div(kNParams, 256), 256, 0, stream, net.params, net.m, net.v, net.part,
+                            net.used, net.loss_part, net.scalars, net.img, 1, net.lr, net.beta1, net.beta2, net.eps, c1,
+                            c2));
   return CKR_OK;
 }
 

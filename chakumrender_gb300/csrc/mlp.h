@@ -46,7 +46,8 @@ struct Net {
   float *scalars = nullptr;  // [0] weight sum of the batch, [1] loss of the last step
   uint8_t *img = nullptr;    // kImgBytes
   int *err = nullptr;
-  uint32_t grid = 0;         // CTAs of the training kernel
+  uint32_t grid = 0;         // most CTAs of the training kernel
+  uint32_t used = 1;         // CTAs of its last launch, which wrote partial sums
   float centre[3] = {0, 0, 0}, scale = 1.0f;
   uint32_t nclusters = 0;
   uint32_t step = 0;

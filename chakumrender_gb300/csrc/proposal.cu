@@ -150,12 +150,12 @@ extern "C" int ckr_internal_proposal_gradients(ckr_proposal *p, const float *rec
   int st = mlp::gradients(p->net, reinterpret_cast<const float4 *>(rec12), n, nullptr, 0, nullptr);
   if (st != CKR_OK) return st;
   CKR_CUDA_TRY(cudaDeviceSynchronize());
-  std::vector<float> part((size_t)p->net.grid * mlp::kNParams), lp(p->net.grid);
+  std::vector<float> part((size_t)p->net.used * mlp::kNParams), lp(p->net.used);
   CKR_CUDA_TRY(cudaMemcpy(part.data(), p->net.part, part.size() * 4, cudaMemcpyDeviceToHost));
   CKR_CUDA_TRY(cudaMemcpy(lp.data(), p->net.loss_part, lp.size() * 4, cudaMemcpyDeviceToHost));
   for (uint32_t j = 0; j < mlp::kNParams; ++j) {
     double g = 0;
-    for (uint32_t c = 0; c < p->net.grid; ++c) g += part[(size_t)c * mlp::kNParams + j];
+    for (uint32_t c = 0; c < p->net.used; ++c) g += part[(size_t)c * mlp::kNParams + j];
     grad[j] = (float)g;
   }
   double l = 0;

@@ -34,9 +34,22 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t base, uint32_t K, uint32_t s)
   return (uint64_t)((start >> 4) & 0x3FFFu) | (lbo << 16) | (sbo << 32) | (1ull << 46);
 }
 
-// Instruction descriptor: D FP32, A and B BF16, both K-major, M x N.
-__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+// Instruction descriptor: D FP32, A and B BF16, M x N; both operands K-major, or
+// (transposed) both MN-major.
+__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N, bool transposed = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (transposed ? 3u << 15 : 0u) | ((N >> 3) << 17) | ((M >> 4) << 24);
+}
+
+// The same memory read the other way: an R x C array stored as above (row r, 8 columns of a
+// core-matrix row contiguous) as the MN-major operand of C rows (MN) and R columns (K), its
+// transpose without a copy.  Core matrices adjacent in MN are 128 bytes apart (the stride
+// byte offset of an MN-major operand), in K C * 16 bytes (its leading byte offset); slice s
+// starts at array row 16 s.  MN extents past C read whatever follows; their accumulator
+// rows are garbage.
+__device__ __forceinline__ uint64_t sdesc_t(uint32_t base, uint32_t C, uint32_t s) {
+  const uint32_t start = base + C * 32u * s;
+  const uint64_t lbo = (C * 16u) >> 4, sbo = 128u >> 4;
+  return (uint64_t)((start >> 4) & 0x3FFFu) | (lbo << 16) | (sbo << 32) | (1ull << 46);
 }
 
 // ---- TMEM allocation (one warp, all lanes) ----
@@ -104,6 +117,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, uint32
   }
   return false;
 }
+
+// ---- asynchronous copy of contiguous global memory into shared memory ----
+// Both addresses 16-byte aligned, bytes a multiple of 16; completes one phase of the
+// mbarrier (initialised with count 1).
+__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void *src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem),
+               "l"(src), "r"(bytes), "r"(mbar)
+               : "memory");
+}
+
+// ---- programmatic dependent launch ----
+// Lets the next kernel of the stream start (one launched with the programmatic
+// attribute; others wait for this grid's end as always).
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Waits until the kernels this launch depends on have ended and their writes are visible.
+__device__ __forceinline__ void wait_dependencies() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- TMEM -> registers: 32 consecutive FP32 columns of this thread's lane ----
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
