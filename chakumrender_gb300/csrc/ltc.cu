@@ -1,14 +1,13 @@
 // ltc.cu — LTC polygon-light shading of a G-buffer (getLightFromMeshSource_Analytic,
 // src/lightSources_CV.cpp:323-333, per pixel).
 //
-// The kernel is FP32-ALU bound (per pixel and emitter triangle: three
+// The kernel is FP32 issue bound (per pixel and emitter triangle: three
 // transformed vertices, horizon clipping, 3-4 edge integrals, for both the
 // specular LTC lobe and the diffuse cosine lobe) and its lanes disagree on the
 // path a triangle takes (above, below or across the horizon), so triangles across
 // the horizon are queued per warp and clipped by all lanes together (k_ltc_shade).
-// CTAs are persistent (three per SM) and stride over pixels; the 64x64 LTC table is
-// read from global memory (two entries per pixel), emitter triangles through the
-// read-only path (every lane of a warp reads the same triangle, a broadcast).
+// CTAs are persistent and stride over pixels; the 64x64 LTC table is
+// read from global memory (two entries per pixel), short emitter lists from shared memory.
 #include <algorithm>
 
 #include "ckr_internal.h"
@@ -19,13 +18,18 @@
 namespace ckr {
 namespace {
 
-constexpr int kLtcTPB = 256, kLtcWarps = kLtcTPB / 32;
-// Deferred triangles per warp and batch of 32 pixels.  256 entries (7.3 KB of shared
-// memory per warp) let three CTAs share an SM: 24 warps at 80 registers with a few
-// spills ran 0.725 ms per 1024^2 frame against 0.846 ms at 512 entries and two CTAs
-// (104 registers); 128 entries at four CTAs (64 registers, 236 bytes of spills) ran
-// 0.966 ms, its queues overflowing into in-place clipping.
+// Blocks of two warps, which share only the emitter list, at 128 registers without spills:
+// 1024^2 pixels and 8 quads take 251 us; four, eight warps a block 250, 254; at ten blocks
+// (96 registers, spills) 258.  Small blocks spread small images: 22 x 771 pixels on 58
+// blocks of eight warps 19.8 us, on 265 blocks of two 10.2.
+constexpr int kLtcTPB = 64, kLtcWarps = kLtcTPB / 32;
+// Deferred triangles per warp and batch of 32 pixels (7.3 KB of shared memory per warp; 384
+// entries at two blocks of 256 threads ran as 256).
 constexpr uint32_t kLtcQueue = 256;
+// Emitter triangles kept in shared memory, 48 bytes each with their radiance: three 16-byte
+// loads a triangle instead of twelve scalar ones (272 -> 266 us, all else alike).  Longer lists
+// are read from global memory.
+constexpr uint32_t kLtcStaged = 64;
 
 // The clipped integrals for a lane whose warp's queue is full.  Out of line: inlined
 // into the classifying loop they pushed it past 128 registers (60 bytes of spills,
@@ -47,8 +51,107 @@ struct GlobalTable {
 struct LtcWarp {
   float px[32][17];          // x (3), n (3), Minv in world space (9); padded against bank conflicts
   float res[kLtcQueue][3];   // a deferred triangle's contribution, colour-weighted
-  uint2 item[kLtcQueue];     // (lane | lobe << 5 | light << 6, previous item of the same lane or ~0)
+  uint2 item[kLtcQueue];     // (lane | light << 5, previous item of the same lane or ~0)
 };
+
+// ---- both lobes at once -------------------------------------------------------------
+// A pair of FP32 numbers in one 64-bit register pair, the specular lobe's in the low half,
+// the diffuse one's in the high half: one FFMA2 does both lobes' multiply-add, each rounded
+// as the scalar instruction rounds it.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float lo2(f2 a) {
+  return __uint_as_float((uint32_t)a);
+}
+__device__ __forceinline__ float hi2(f2 a) {
+  return __uint_as_float((uint32_t)(a >> 32));
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// A corner of an emitter triangle as the two lobes see it: unit vectors (specular in the
+// LTC's canonical space), and its height over the horizon of each (the specular one before
+// normalisation, as ltc_spec_case tests it).
+struct Corner {
+  f2 x, y, z;
+  float hs, hd;
+};
+
+__device__ __forceinline__ Corner corner(F3 P, F3 x, F3 n, const M3f &minv) {
+  const F3 d = P - x, q = mul(minv, d);
+  const f2 X = pk(q.x, d.x), Y = pk(q.y, d.y), Z = pk(q.z, d.z);
+  // dot() and normalize(), pairwise and in their order of rounding: the edge factor
+  // amplifies a last bit of these where an edge passes close to the point.
+  const f2 nn = fma2(Z, Z, fma2(X, X, mul2(Y, Y)));
+  const f2 r = pk(rsqrtf(lo2(nn)), rsqrtf(hi2(nn)));
+  Corner c;
+  c.x = mul2(X, r);
+  c.y = mul2(Y, r);
+  c.z = mul2(Z, r);
+  c.hs = q.z;
+  c.hd = dot(f3(hi2(c.x), hi2(c.y), hi2(c.z)), n);
+  return c;
+}
+
+// theta_over_sin's coefficients, negated, in pairs.
+__constant__ float2 c_theta[10] = {
+    {-1.570796251296997f, -1.570796251296997f},
+    {0.9999964833259583f, 0.9999964833259583f},
+    {-0.7852754592895508f, -0.7852754592895508f},
+    {0.6649839878082275f, 0.6649839878082275f},
+    {-0.5770568251609802f, -0.5770568251609802f},
+    {0.48246079683303833f, 0.48246079683303833f},
+    {-0.35151180624961853f, -0.35151180624961853f},
+    {0.19518974423408508f, 0.19518974423408508f},
+    {-0.06951962411403656f, -0.06951962411403656f},
+    {0.011529042385518551f, 0.011529042385518551f}};
+
+// The edge integrals of both lobes (integrate_edge_z, integrate_edge; theta_over_sin's
+// polynomial in pairs).
+__device__ __forceinline__ void edge2(const Corner &a, const Corner &b, F3 n, float &s, float &d) {
+  const f2 cc = fma2(a.z, b.z, fma2(a.x, b.x, mul2(a.y, b.y)));
+  const float cs = lo2(cc), cd = hi2(cc);
+  const float us = fminf(fabsf(cs), 1.0f), ud = fminf(fabsf(cd), 1.0f);
+  const f2 u = pk(us, ud);
+  const f2 *k = reinterpret_cast<const f2 *>(c_theta);
+  f2 g = k[9];  // the negated polynomial
+#pragma unroll
+  for (int i = 8; i >= 0; --i) g = fma2(g, u, k[i]);
+  // Both cases of theta_over_sin: some lane of a warp nearly always has an obtuse angle.
+  const f2 one = pk(1.0f, 1.0f), q = mul2(fma2(u, pk(-1.0f, -1.0f), one), fma2(u, one, one));
+  const f2 obtuse = fma2(pk(kPi, kPi), pk(rsqrtf(lo2(q)), rsqrtf(hi2(q))), g);
+  const float gs = cs >= 0.0f ? -lo2(g) : lo2(obtuse), gd = cd >= 0.0f ? -hi2(g) : hi2(obtuse);
+  const float ax = hi2(a.x), ay = hi2(a.y), az = hi2(a.z), bx = hi2(b.x), by = hi2(b.y), bz = hi2(b.z);
+  s = (lo2(a.x) * lo2(b.y) - lo2(a.y) * lo2(b.x)) * gs;
+  d = dot(cross(f3(ax, ay, az), f3(bx, by, bz)), n) * gd;
+}
+
+// Least and greatest of three numbers, NaN if one is.
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
+  float r;
+  asm("{\n\t.reg .f32 t;\n\tmin.NaN.f32 t, %1, %2;\n\tmin.NaN.f32 %0, t, %3;\n\t}" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float r;
+  asm("{\n\t.reg .f32 t;\n\tmax.NaN.f32 t, %1, %2;\n\tmax.NaN.f32 %0, t, %3;\n\t}" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// Whether two corners of the emitter list are the same point.
+__device__ __forceinline__ bool same(F3 a, F3 b) { return a.x == b.x && a.y == b.y && a.z == b.z; }
 
 // getLightFromMeshSource_Analytic per pixel, one pixel per lane.  Per emitter
 // triangle and lobe a lane settles the triangles wholly above or below its horizon
@@ -57,7 +160,17 @@ struct LtcWarp {
 // the few lanes that clip hold up the rest.  Each lane adds its queued terms in a
 // fixed order (newest first), so the result does not depend on scheduling.  A full
 // queue falls back to clipping in place.
-__global__ void __launch_bounds__(kLtcTPB, 3) k_ltc_shade(const float4 *__restrict__ gbuf, uint32_t npx,
+// FP32 issue bound.  The two lobes run in pairs (FFMA2, above), and two consecutive
+// triangles that share the edge from their first corner, (a, p, m) and (a, m, q) in either
+// order -- a quad, a fan; what polygon emitters are made of -- take their common corners and
+// edge once: 4 corners and 5 edges instead of 6 and 6.  The test is the same for all lanes.
+// Triangles across the horizon are queued by lobe, so that a warp clips one lobe at a time,
+// and clipped without branches (clip_edges); with one mixed queue and a branch per crossed
+// edge the clipping was half of all instructions.  1024^2 pixels, 8 quads: 370 -> 251 us,
+// warp instructions 344 M -> 249 M, active lanes 20.0 -> 26.7 before
+// the emitter list moved to shared memory.
+template <bool STAGED>
+__global__ void __launch_bounds__(kLtcTPB, 8) k_ltc_shade(const float4 *__restrict__ gbuf, uint32_t npx,
                                                        const float *__restrict__ light_tri9,
                                                        const float *__restrict__ light_rgb, uint32_t nlight,
                                                        float *__restrict__ rgb, const LtcEntry *__restrict__ table) {
@@ -65,14 +178,27 @@ __global__ void __launch_bounds__(kLtcTPB, 3) k_ltc_shade(const float4 *__restri
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   LtcWarp &W = reinterpret_cast<LtcWarp *>(ltc_smem)[warp];
   const GlobalTable tab{table};
-  auto light = [&](uint32_t k, F3 &A, F3 &B, F3 &C, float *c) {
-    const float *t = light_tri9 + 9 * (size_t)k;
-    A = f3(__ldg(t), __ldg(t + 1), __ldg(t + 2));
-    B = f3(__ldg(t + 3), __ldg(t + 4), __ldg(t + 5));
-    C = f3(__ldg(t + 6), __ldg(t + 7), __ldg(t + 8));
-    c[0] = __ldg(light_rgb + 3 * k);
-    c[1] = __ldg(light_rgb + 3 * k + 1);
-    c[2] = __ldg(light_rgb + 3 * k + 2);
+  // Emitter triangle k and its radiance.
+  __shared__ float4 staged[STAGED ? 3 * kLtcStaged : 1];  // (A, r) (B, g) (C, b)
+  if constexpr (STAGED) {
+    for (uint32_t i = threadIdx.x; i < 3 * nlight; i += kLtcTPB)
+      staged[i] = make_float4(light_tri9[3 * i], light_tri9[3 * i + 1], light_tri9[3 * i + 2], light_rgb[i]);
+    __syncthreads();
+  }
+  auto tri = [&](uint32_t k, F3 &A, F3 &B, F3 &C, F3 &col) {
+    if constexpr (STAGED) {
+      const float4 a = staged[3 * k], b = staged[3 * k + 1], c = staged[3 * k + 2];
+      A = f3(a.x, a.y, a.z);
+      B = f3(b.x, b.y, b.z);
+      C = f3(c.x, c.y, c.z);
+      col = f3(a.w, b.w, c.w);
+    } else {
+      const float *t = light_tri9 + 9 * (size_t)k, *c = light_rgb + 3 * (size_t)k;
+      A = f3(__ldg(t), __ldg(t + 1), __ldg(t + 2));
+      B = f3(__ldg(t + 3), __ldg(t + 4), __ldg(t + 5));
+      C = f3(__ldg(t + 6), __ldg(t + 7), __ldg(t + 8));
+      col = f3(__ldg(c), __ldg(c + 1), __ldg(c + 2));
+    }
   };
   const float inv2pi = 1.0f / (2.0f * kPi);
   for (uint32_t base = (blockIdx.x * kLtcWarps + warp) * 32u; base < npx; base += gridDim.x * (uint32_t)kLtcTPB) {
@@ -97,64 +223,107 @@ __global__ void __launch_bounds__(kLtcTPB, 3) k_ltc_shade(const float4 *__restri
     mine[3] = n.x; mine[4] = n.y; mine[5] = n.z;
     for (int i = 0; i < 9; ++i) mine[6 + i] = minv.a[i];
     float s3[3] = {0.f, 0.f, 0.f}, d3[3] = {0.f, 0.f, 0.f};
-    uint32_t head = ~0u, count = 0;  // count: the same in every lane
-    for (uint32_t k = 0; k < nlight; ++k) {
-      F3 A, B, C;
-      float c[3];
-      light(k, A, B, C, c);
-      float s = 0.f, d = 0.f;
-      int cs = 0, cd = 0;
-      if (active) {
-        cs = ltc_spec_case(A, B, C, x, minv, s);
-        cd = ltc_diffuse_case(A, B, C, n, x, d);
-      }
-      for (int j = 0; j < 3; ++j) {
-        s3[j] += c[j] * s;
-        d3[j] += c[j] * d;
-      }
+    // Queued triangles: specular ones from the front, diffuse ones from the back, so that a
+    // warp clips one lobe at a time.  The counts are the same in every lane.
+    uint32_t head = ~0u, count[2] = {0, 0};
+    // Adds triangle k: the lobes' integrals `is`, `id` if it is above their horizon; across
+    // it, its queue entries.
+    auto add = [&](uint32_t k, F3 col, const Corner &a, const Corner &b, const Corner &c, float is, float id) {
+      const float r = col.x, g = col.y, bl = col.z;
+      // A NaN height is neither above nor below: queued.
+      const bool us = min3_nan(a.hs, b.hs, c.hs) > 0.f, ud = min3_nan(a.hd, b.hd, c.hd) > 0.f;
+      const float s = us ? fabsf(is) : 0.f, d = ud ? fabsf(id) : 0.f;
+      s3[0] += r * s; s3[1] += g * s; s3[2] += bl * s;
+      d3[0] += r * d; d3[1] += g * d; d3[2] += bl * d;
+      const bool qs = active && !us && !(max3_nan(a.hs, b.hs, c.hs) < 0.f);
+      const bool qd = active && !ud && !(max3_nan(a.hd, b.hd, c.hd) < 0.f);
+#pragma unroll
       for (uint32_t lobe = 0; lobe < 2; ++lobe) {
-        const bool want = (lobe ? cd : cs) < 0;
+        const bool want = lobe ? qd : qs;
         const unsigned m = __ballot_sync(0xffffffffu, want);
-        const uint32_t slot = count + (uint32_t)__popc(m & ((1u << lane) - 1u));
+        if (m == 0) continue;
+        const uint32_t rank = count[lobe] + (uint32_t)__popc(m & ((1u << lane) - 1u));
         if (want) {
-          if (slot < kLtcQueue) {
-            W.item[slot] = make_uint2(lane | lobe << 5 | k << 6, head);
+          if (rank + count[lobe ^ 1u] < kLtcQueue) {
+            const uint32_t slot = lobe ? kLtcQueue - 1u - rank : rank;
+            W.item[slot] = make_uint2(lane | k << 5, head);
             head = slot;
-          } else if (lobe) {
-            const float v = clipped_diffuse_here(A, B, C, n, x);
-            for (int j = 0; j < 3; ++j) d3[j] += c[j] * v;
           } else {
-            const float v = clipped_spec_here(A, B, C, x, minv);
-            for (int j = 0; j < 3; ++j) s3[j] += c[j] * v;
+            F3 A, B, C, unused;
+            tri(k, A, B, C, unused);
+            const float v = lobe ? clipped_diffuse_here(A, B, C, n, x) : clipped_spec_here(A, B, C, x, minv);
+            float *acc = lobe ? d3 : s3;
+            acc[0] += r * v; acc[1] += g * v; acc[2] += bl * v;
           }
         }
-        count += (uint32_t)__popc(m);
+        count[lobe] = min(count[lobe] + (uint32_t)__popc(m), kLtcQueue - count[lobe ^ 1u]);
+      }
+    };
+    for (uint32_t k = 0; k < nlight;) {
+      F3 A, B, C, A2, B2, C2, col, col2;
+      tri(k, A, B, C, col);
+      uint32_t first = k, second = k;  // second == first: no pair
+      F3 pp = B, pm = C, pq = C;
+      if (k + 1 < nlight) {
+        tri(k + 1, A2, B2, C2, col2);
+        if (same(A, A2)) {
+          if (same(C, B2)) {
+            second = k + 1;
+            pq = C2;
+          } else if (same(B, C2)) {
+            first = k + 1;
+            pp = B2;
+            pm = C2;
+            pq = C;
+            const F3 swap = col;
+            col = col2;
+            col2 = swap;
+          }
+        }
+      }
+      const Corner a = corner(A, x, n, minv), b = corner(pp, x, n, minv), c = corner(pm, x, n, minv);
+      float s0, d0, s1, d1, sm, dm;
+      edge2(a, b, n, s0, d0);
+      edge2(b, c, n, s1, d1);
+      edge2(c, a, n, sm, dm);
+      add(first, col, a, b, c, s0 + s1 + sm, d0 + d1 + dm);
+      if (first != second) {
+        const Corner q = corner(pq, x, n, minv);
+        edge2(c, q, n, s0, d0);
+        edge2(q, a, n, s1, d1);
+        add(second, col2, a, c, q, s0 + s1 - sm, d0 + d1 - dm);
+        k += 2;
+      } else {
+        k += 1;
       }
     }
     __syncwarp();
     // The warp's queued triangles, every lane taking the next one.
-    const uint32_t nq = count < kLtcQueue ? count : kLtcQueue;
-    for (uint32_t i = lane; i < nq; i += 32) {
-      const uint2 it = W.item[i];
-      const uint32_t pl = it.x & 31u, k = it.x >> 6;
-      const float *q = W.px[pl];
-      F3 A, B, C;
-      float c[3];
-      light(k, A, B, C, c);
-      const F3 qx = f3(q[0], q[1], q[2]);
-      float v;
-      if ((it.x >> 5) & 1u) {
-        v = ltc_diffuse_clipped(A, B, C, f3(q[3], q[4], q[5]), qx);
-      } else {
-        M3f qm;
-        for (int j = 0; j < 9; ++j) qm.a[j] = q[6 + j];
-        v = ltc_spec_clipped(A, B, C, qx, qm);
+#pragma unroll
+    for (uint32_t lobe = 0; lobe < 2; ++lobe)
+      for (uint32_t i = lane; i < count[lobe]; i += 32) {
+        const uint32_t slot = lobe ? kLtcQueue - 1u - i : i;
+        const uint2 it = W.item[slot];
+        const uint32_t k = it.x >> 5;
+        const float *q = W.px[it.x & 31u];
+        F3 A, B, C, col;
+        tri(k, A, B, C, col);
+        const F3 qx = f3(q[0], q[1], q[2]);
+        float v;
+        if (lobe) {
+          v = ltc_diffuse_clipped(A, B, C, f3(q[3], q[4], q[5]), qx);
+        } else {
+          M3f qm;
+          for (int j = 0; j < 9; ++j) qm.a[j] = q[6 + j];
+          v = ltc_spec_clipped(A, B, C, qx, qm);
+        }
+        W.res[slot][0] = col.x * v;
+        W.res[slot][1] = col.y * v;
+        W.res[slot][2] = col.z * v;
       }
-      for (int j = 0; j < 3; ++j) W.res[i][j] = c[j] * v;
-    }
     __syncwarp();
     for (uint32_t i = head; i != ~0u; i = W.item[i].y) {
-      if ((W.item[i].x >> 5) & 1u) {
+      if (i >= count[0]) {
         for (int j = 0; j < 3; ++j) d3[j] += W.res[i][j];
       } else {
         for (int j = 0; j < 3; ++j) s3[j] += W.res[i][j];
@@ -298,19 +467,21 @@ extern "C" int ckr_ltc_shade(const float *gbuf, uint32_t npx, const float *light
   if (!table) return st;
   if (nlight >= (1u << 26)) return CKR_ERR_TOO_LARGE;  // light index in a queue item
   const size_t smem = kLtcWarps * sizeof(LtcWarp);
+  const auto fn = nlight <= kLtcStaged ? k_ltc_shade<true> : k_ltc_shade<false>;
   static bool attr_set[64] = {false};
   int dev = 0, sms = 0, per_sm = 0;
   CKR_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    CKR_CUDA_TRY(cudaFuncSetAttribute(k_ltc_shade, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (const void *k : {(const void *)k_ltc_shade<true>, (const void *)k_ltc_shade<false>})
+      CKR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[dev] = true;
   }
   CKR_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  CKR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ltc_shade, kLtcTPB, smem));
+  CKR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLtcTPB, smem));
   if (per_sm < 1) return CKR_ERR_CUDA;
   int grid = (int)std::min<uint64_t>(ceil_div(npx, kLtcTPB), (uint64_t)sms * per_sm);
-  k_ltc_shade<<<grid, kLtcTPB, smem, (cudaStream_t)stream>>>(reinterpret_cast<const float4 *>(gbuf), npx, light_tri9,
-                                                               light_rgb, nlight, rgb, table);
+  fn<<<grid, kLtcTPB, smem, (cudaStream_t)stream>>>(reinterpret_cast<const float4 *>(gbuf), npx, light_tri9, light_rgb,
+                                                    nlight, rgb, table);
   CKR_CUDA_TRY(cudaGetLastError());
   return CKR_OK;
 }

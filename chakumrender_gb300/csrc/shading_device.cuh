@@ -435,111 +435,58 @@ SHD float integrate_edge_z(F3 v1, F3 v2) { return (v1.x * v2.y - v1.y * v2.x) * 
 // positive exactly when -1 < d < 0 (and, for CA, A.x != C.x).  Testing d
 // directly gives the same answer without the cancellation that makes the
 // product round to zero in FP32 when a vertex lies within ~1e-4 of the plane.
-SHD bool edge_crossed(float d) { return d > -1.0f && d < 0.0f; }
+// d = p / n is between -1 and 0 exactly when p and n differ in sign and |p| < |n|
+// (a quotient of two FP32 numbers with |p| < |n| is at most 1 - 2^-24, which rounds to
+// itself or below), so only the edges that are used are divided.
+SHD bool edge_crossed(float p, float n) { return (p < 0.f) != (n < 0.f) && p != 0.f && fabsf(p) < fabsf(n); }
 
-// Records a clipped edge segment: the first two points go to q0, q1, the next
-// two to q2, q3 (clipTriangle's clip[idx++] sequence without a local array).
+// The clipped polygon: clipTriangle's clip[idx++] sequence, the segments of the first two
+// crossed edges in the order AB, BC, CA.
 struct Clip4 {
   F3 q0, q1, q2, q3;
-  int idx;
-  SHD void push(F3 a, F3 b) {
-    if (idx == 0) {
-      q0 = a;
-      q1 = b;
-    } else if (idx == 2) {
-      q2 = a;
-      q3 = b;
-    }
-    idx += 2;
-  }
 };
 
-// clipTriangle against the plane through P with normal n, general variant
-// (src/lightSources_CV.cpp:28-130), including its test on edge CA that looks
-// at x coordinates only (:101-102).
-SHD bool clip_triangle(F3 A, F3 B, F3 C, F3 n, F3 P, float nA, float nB, float nC, Clip4 &clip) {
+SHD F3 pick(bool c, F3 a, F3 b) { return f3(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z); }
+
+// Segment of the crossed edge PQ: from the crossing to Q when P is below the plane, else
+// from P to the crossing.
+SHD void clip_segment(F3 P, F3 Q, float p, float n, bool below, F3 &a, F3 &b) {
+  const float d = p / n;
+  const F3 i = (P - Q) * d + P;
+  a = pick(below, i, P);
+  b = pick(below, Q, i);
+}
+
+// The part of clipTriangle after its plane distances (src/lightSources_CV.cpp:44-130,
+// 145-219), without branches: lanes of a warp cross different edges.  For edge PQ, n is the
+// height of P over Q and p the plane's height over P; below[]: the corner is below.
+// Edges (nearly) in parallel with the plane are not crossed, and one in the plane ends
+// the clipping; edge CA needs corners of different x (the reference's test, :101-102).
+SHD bool clip_edges(F3 A, F3 B, F3 C, float pA, float pB, float pC, float nAB, float nBC, float nCA, bool bA, bool bB,
+                    bool bC, Clip4 &clip) {
   const float eps = 1e-15f;
-  int hits = 0;
-  clip.idx = 0;
-  F3 dAB = A - B, dBC = B - C, dCA = C - A;
-  float nAB = dot(n, dAB), nBC = dot(n, dBC), nCA = dot(n, dCA);
-  float pA = dot(n, P - A), pB = dot(n, P - B), pC = dot(n, P - C);
-  if (nAB * nAB > eps) {
-    float d = pA / nAB;
-    F3 i = dAB * d + A;
-    if (edge_crossed(d)) {
-      ++hits;
-      if (nA < 0.f) clip.push(i, B);
-      else clip.push(A, i);
-    }
-  } else if (pA * pA < eps) {
-    return false;
-  }
-  if (nBC * nBC > eps) {
-    float d = pB / nBC;
-    F3 i = dBC * d + B;
-    if (edge_crossed(d)) {
-      ++hits;
-      if (nB < 0.f) clip.push(i, C);
-      else clip.push(B, i);
-    }
-  } else if (pB * pB < eps) {
-    return false;
-  }
-  if (nCA * nCA > eps) {
-    float d = pC / nCA;
-    F3 i = dCA * d + C;
-    if (edge_crossed(d) && A.x != C.x) {
-      ++hits;
-      if (nC < 0.f) clip.push(i, A);
-      else clip.push(C, i);
-    }
-  } else if (pC * pC < eps) {
-    return false;
-  }
-  return hits > 1;
+  const bool sAB = nAB * nAB > eps, sBC = nBC * nBC > eps, sCA = nCA * nCA > eps;
+  const bool dead = (!sAB && pA * pA < eps) || (!sBC && pB * pB < eps) || (!sCA && pC * pC < eps);
+  const bool hAB = sAB && edge_crossed(pA, nAB), hBC = sBC && edge_crossed(pB, nBC),
+             hCA = sCA && edge_crossed(pC, nCA) && A.x != C.x;
+  // First segment: of AB, else of BC; second: of BC if AB is crossed too, else of CA.
+  const bool two_bc = hAB && hBC;
+  clip_segment(pick(hAB, A, B), pick(hAB, B, C), hAB ? pA : pB, hAB ? nAB : nBC, hAB ? bA : bB, clip.q0, clip.q1);
+  clip_segment(pick(two_bc, B, C), pick(two_bc, C, A), two_bc ? pB : pC, two_bc ? nBC : nCA, two_bc ? bB : bC, clip.q2,
+               clip.q3);
+  return !dead && (int)hAB + (int)hBC + (int)hCA > 1;
+}
+
+// clipTriangle against the plane through P with normal n, general variant
+// (src/lightSources_CV.cpp:28-130); nA, nB, nC: the corners' heights over it by sign.
+SHD bool clip_triangle(F3 A, F3 B, F3 C, F3 n, F3 P, float nA, float nB, float nC, Clip4 &clip) {
+  return clip_edges(A, B, C, dot(n, P - A), dot(n, P - B), dot(n, P - C), dot(n, A - B), dot(n, B - C), dot(n, C - A),
+                    nA < 0.f, nB < 0.f, nC < 0.f, clip);
 }
 
 // Same against the plane z = 0 (src/lightSources_CV.cpp:133-219).
-SHD bool clip_triangle_z(F3 A, F3 B, F3 C, float nA, float nB, float nC, Clip4 &clip) {
-  const float eps = 1e-15f;
-  int hits = 0;
-  clip.idx = 0;
-  F3 dAB = A - B, dBC = B - C, dCA = C - A;
-  if (dAB.z * dAB.z > eps) {
-    float d = -A.z / dAB.z;
-    F3 i = dAB * d + A;
-    if (edge_crossed(d)) {
-      ++hits;
-      if (nA < 0.f) clip.push(i, B);
-      else clip.push(A, i);
-    }
-  } else if (A.z * A.z < eps) {
-    return false;
-  }
-  if (dBC.z * dBC.z > eps) {
-    float d = -B.z / dBC.z;
-    F3 i = dBC * d + B;
-    if (edge_crossed(d)) {
-      ++hits;
-      if (nB < 0.f) clip.push(i, C);
-      else clip.push(B, i);
-    }
-  } else if (B.z * B.z < eps) {
-    return false;
-  }
-  if (dCA.z * dCA.z > eps) {
-    float d = -C.z / dCA.z;
-    F3 i = dCA * d + C;
-    if (edge_crossed(d) && A.x != C.x) {
-      ++hits;
-      if (nC < 0.f) clip.push(i, A);
-      else clip.push(C, i);
-    }
-  } else if (C.z * C.z < eps) {
-    return false;
-  }
-  return hits > 1;
+SHD bool clip_triangle_z(F3 A, F3 B, F3 C, Clip4 &clip) {
+  return clip_edges(A, B, C, -A.z, -B.z, -C.z, A.z - B.z, B.z - C.z, C.z - A.z, A.z < 0.f, B.z < 0.f, C.z < 0.f, clip);
 }
 
 // |polygon integral| of one emitter triangle for the cosine lobe about n at x
@@ -563,12 +510,12 @@ SHD float ltc_diffuse_clipped(F3 A, F3 B, F3 C, F3 n, F3 x) {
   F3 e1 = normalize(A - x), e2 = normalize(B - x), e3 = normalize(C - x);
   float nA = dot(e1, n), nB = dot(e2, n), nC = dot(e3, n);
   Clip4 clip;
-  clip.q0 = clip.q1 = clip.q2 = clip.q3 = f3(0, 0, 0);
-  if (!clip_triangle(A, B, C, n, x, nA, nB, nC, clip)) return 0.0f;
+  const bool ok = clip_triangle(A, B, C, n, x, nA, nB, nC, clip);
   F3 c0 = normalize(clip.q0 - x), c1 = normalize(clip.q1 - x), c2 = normalize(clip.q2 - x),
      c3 = normalize(clip.q3 - x);
-  return fabsf(integrate_edge(c0, c1, n) + integrate_edge(c1, c2, n) + integrate_edge(c2, c3, n) +
-               integrate_edge(c3, c0, n));
+  const float v = fabsf(integrate_edge(c0, c1, n) + integrate_edge(c1, c2, n) + integrate_edge(c2, c3, n) +
+                        integrate_edge(c3, c0, n));
+  return ok ? v : 0.0f;
 }
 
 SHD float ltc_diffuse_tri(F3 A, F3 B, F3 C, F3 n, F3 x) {
@@ -595,12 +542,12 @@ SHD int ltc_spec_case(F3 A, F3 B, F3 C, F3 x, const M3f &minv, float &s) {
 SHD float ltc_spec_clipped(F3 A, F3 B, F3 C, F3 x, const M3f &minv) {
   F3 e1 = mul(minv, A - x), e2 = mul(minv, B - x), e3 = mul(minv, C - x);
   Clip4 clip;
-  clip.q0 = clip.q1 = clip.q2 = clip.q3 = f3(0, 0, 0);
-  if (!clip_triangle_z(e1, e2, e3, e1.z / length(e1), e2.z / length(e2), e3.z / length(e3), clip)) return 0.0f;
+  const bool ok = clip_triangle_z(e1, e2, e3, clip);
   F3 c0 = normalize(clip.q0), c1 = normalize(clip.q1), c2 = normalize(clip.q2),
      c3 = normalize(clip.q3);
-  return fabsf(integrate_edge_z(c0, c1) + integrate_edge_z(c1, c2) + integrate_edge_z(c2, c3) +
-               integrate_edge_z(c3, c0));
+  const float v = fabsf(integrate_edge_z(c0, c1) + integrate_edge_z(c1, c2) + integrate_edge_z(c2, c3) +
+                        integrate_edge_z(c3, c0));
+  return ok ? v : 0.0f;
 }
 
 SHD float ltc_spec_tri(F3 A, F3 B, F3 C, F3 x, const M3f &minv) {
