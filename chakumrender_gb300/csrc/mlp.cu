@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "ckr_internal.h"
@@ -137,6 +138,15 @@ __device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t *dst, uint
   *reinterpret_cast<uint4 *>(dst + tc::kmaj(t, 72, kHidK)) = make_uint4(0u, 0u, 0u, 0u);
 }
 
+// exp(z) for z in [-80, 80] as 2^(z log2 e): the result is a normal number, so the flushing
+// form of the instruction does, without the scaling around it that __expf needs for
+// denormal results (two multiplies and a compare of every logit).
+__device__ __forceinline__ float exp_80(float z) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmul_rn(z, 1.4426950408889634f)));
+  return r;
+}
+
 // exp(z) over the logits of row t when all 64 are clusters, with z clamped to
 // [-80, 80] so that neither the terms nor their sum leave FP32's range (the
 // softmax does not change for logits inside that range); returns the sum.
@@ -146,7 +156,7 @@ __device__ __forceinline__ float softmax_exp64(uint32_t taddr, float *p) {
   float sum = 0.f;
 #pragma unroll
   for (int j = 0; j < 64; ++j) {
-    p[j] = __expf(fminf(fmaxf(p[j], -80.f), 80.f));
+    p[j] = exp_80(fminf(fmaxf(p[j], -80.f), 80.f));
     sum += p[j];
   }
   return sum;
@@ -222,7 +232,7 @@ constexpr uint32_t kGroups = 2, kInferTPB = 128 * kGroups;
 struct SmemInfer {
   uint8_t w[kImgForward];
   uint8_t a[kGroups][128 * kIn * 2];
-  uint64_t mbar[kGroups];
+  uint64_t mbar[kGroups], mbar_w;
   uint32_t tmem;
   int abort[kGroups];
 };
@@ -282,18 +292,19 @@ __device__ __forceinline__ void path_row(const PathRows &pr, const PathGather &g
   r2 = make_float4(S.wo.x, S.wo.y, S.wo.z, 0.f);
 }
 
-template <bool PATHS>
-__global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(const float4 *__restrict__ rec, PathRows pr, uint32_t n_max,
-                                                         const uint32_t *n_dev, uint32_t n_off,
+// The renderer's queue entries to selection CDFs.
+__global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(PathRows pr, uint32_t n_max, const uint32_t *n_dev,
                                                          const uint8_t *__restrict__ img, Params p, float delta,
-                                                         __half *__restrict__ probs, uint16_t *__restrict__ cdf16,
-                                                         int *err) {
+                                                         uint16_t *__restrict__ cdf16, int *err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   SmemInfer &S = *reinterpret_cast<SmemInfer *>(smem_raw);
   const uint32_t g = threadIdx.x >> 7, t = threadIdx.x & 127u, warp = threadIdx.x >> 5;
-  for (uint32_t i = threadIdx.x; i < kImgForward / 16; i += kInferTPB)
-    reinterpret_cast<uint4 *>(S.w)[i] = reinterpret_cast<const uint4 *>(img)[i];
-  const uint32_t mbar = tc::smem_u32(&S.mbar[g]);
+  // The weights by one bulk copy, waited for before a group's first MMA.
+  const uint32_t mbar = tc::smem_u32(&S.mbar[g]), mbar_w = tc::smem_u32(&S.mbar_w);
+  if (threadIdx.x == 0) {
+    tc::mbar_init(mbar_w, 1);
+    tc::bulk_load(tc::smem_u32(S.w), img, kImgForward, mbar_w);
+  }
   if (t == 0) {
     tc::mbar_init(mbar, 1);
     S.abort[g] = 0;
@@ -304,37 +315,38 @@ __global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(const float4 *__rest
   tc::fence_after_sync();
   // Warp w reads TMEM lanes 32 (w % 4) .. +31; group g owns columns 64 g .. +63.
   const uint32_t tmem = S.tmem + 64u * g, lane_addr = tmem + (((warp & 3u) * 32u) << 16);
-  const uint32_t n = rows(n_max, n_dev, n_off);
+  const uint32_t n = rows(n_max, n_dev, 0);
   uint8_t *A = S.a[g];
   const uint32_t a_addr = tc::smem_u32(A), w_addr = tc::smem_u32(S.w);
   uint32_t phase = 0;
   const uint32_t stride = gridDim.x * kGroups;
-  // PATHS: the gather of the next tile's rows runs one tile ahead -- its queue load
+  // The gather of the next tile's rows runs one tile ahead -- its queue load
   // from the start of this tile's MMA chain, its hit and ray loads from the second
   // layer, its triangle's normal and material (ShadeView::tri_nm) during the softmax --
   // so that a row's inputs are in registers when its tile starts (spheres still
   // read the scene through make_surface).  Two CTAs per SM: 128 registers.
   PathGather cur{}, nxt{};
-  if (PATHS) {
-    gather_slot(pr, (blockIdx.x * kGroups + g) * 128u + t, n, cur);
-    gather_hit(pr, cur);
-    gather_na(pr, cur);
-  }
+  const uint32_t row0 = (blockIdx.x * kGroups + g) * 128u + t;
+  gather_slot(pr, row0, n, cur);
+  gather_hit(pr, cur);
+  gather_na(pr, cur);
+  bool ok = true;
   for (uint32_t tile = blockIdx.x * kGroups + g; tile * 128u < n; tile += stride) {
     const uint32_t row = tile * 128u + t;
-    float4 r0 = make_float4(0, 0, 0, 0), r1 = r0, r2 = r0;
-    if (PATHS) {
-      path_row(pr, cur, r0, r1, r2);
-      gather_slot(pr, (tile + stride) * 128u + t, n, nxt);
-    } else if (row < n) {
-      r0 = rec[3 * (size_t)row];
-      r1 = rec[3 * (size_t)row + 1];
-      r2 = rec[3 * (size_t)row + 2];
-    }
+    float4 r0, r1, r2;
+    path_row(pr, cur, r0, r1, r2);
+    gather_slot(pr, (tile + stride) * 128u + t, n, nxt);
     write_features(A, t, r0, r1, r2, p);
-    bool ok = true;
+    if (row == row0 && t == 0 && !tc::mbar_wait(mbar_w, 0, kWaitTries)) {
+      S.abort[g] = 1;
+      atomicExch(err, CKR_ERR_ITERATION_LIMIT);
+    }
     for (int l = 0; l < 4 && ok; ++l) {
       sync_for_mma(g);
+      if (S.abort[g]) {
+        ok = false;  // the weights never arrived
+        break;
+      }
       if (t == 0 && !(p.stall_tries && l == 0)) {
         tc::fence_after_sync();
         if (l == 0) issue(tmem, a_addr, w_addr + kImgW1, kIn, 0);
@@ -343,14 +355,14 @@ __global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(const float4 *__rest
       }
       ok = wait_mma(g, mbar, phase, &S.abort[g], err, p.stall_tries ? p.stall_tries : kWaitTries);
       if (ok && l < 3) epilogue_relu(lane_addr, A, t);
-      if (PATHS && l == 1) gather_hit(pr, nxt);
+      if (l == 1) gather_hit(pr, nxt);
     }
     if (!ok) break;
-    if (PATHS) gather_na(pr, nxt);
+    gather_na(pr, nxt);
     float e[64];
     const bool full = p.nclusters == 64;
     const float sum = full ? softmax_exp64(lane_addr, e) : softmax_exp(lane_addr, p.nclusters, e);
-    if (row < n && cdf16 && full) {
+    if (row < n && full) {
       const float unif = delta / 64.0f, keep = (1.0f - delta) / sum;
       float run = 0.f;
       uint32_t w[32];
@@ -365,7 +377,7 @@ __global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(const float4 *__rest
       uint4 *dst = reinterpret_cast<uint4 *>(cdf16 + 64 * (size_t)row);
 #pragma unroll
       for (int q = 0; q < 8; ++q) dst[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-    } else if (row < n && cdf16) {
+    } else if (row < n) {
       // Selection mixture (1 - delta) softmax + delta / C as a 16-bit cumulative
       // table: entry j = round(65535 * sum_{i <= j} q_i), the last cluster's 65535.
       const float unif = delta / (float)p.nclusters, keep = (1.0f - delta) / sum;
@@ -383,11 +395,142 @@ __global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(const float4 *__rest
 #pragma unroll
       for (int q = 0; q < 8; ++q) dst[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
     }
-    if (row < n && probs) {
-      const float inv = 1.0f / sum;
-      uint4 *dst = reinterpret_cast<uint4 *>(probs + 64 * (size_t)row);
+    cur = nxt;
+    tc::fence_before_sync();
+    group_sync(g);
+  }
+  tc::mbar_wait(mbar_w, 0, kWaitTries);  // a group without a tile: the copy has to land before the block ends
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(S.tmem, 64 * kGroups);
+}
+
+// ---- inference on records ----------------------------------------------------------
+// Latency bound: what a tile takes is a chain of features, four MMA groups and their
+// epilogues, so as many tiles as fit run side by side: seven groups of 128 threads in one
+// block per SM (shared memory: the weights and 24 KB a group; 72 registers, which the softmax
+// meets by reading its logits from tensor memory once for the sum and again for the
+// probabilities).  The next tile's records load during this one, the weights come by one bulk
+// copy.  262,144 records: 39.0 us at two blocks of two groups and 128 registers, 36.6 with
+// the copy and the early loads (two threads a row at 64 registers: 36.5), 33.1 so.
+constexpr uint32_t kRecGroups = 7, kRecTPB = 128 * kRecGroups;
+
+struct SmemInferRec {
+  uint8_t w[kImgForward];
+  uint8_t a[kRecGroups][128 * kIn * 2];
+  uint64_t mbar[kRecGroups], mbar_w;
+  uint32_t tmem;
+  int abort[kRecGroups];
+};
+
+__device__ __forceinline__ void rec_group_sync(uint32_t g) {
+  asm volatile("bar.sync %0, 128;" ::"r"(g + 1u) : "memory");
+}
+
+__global__ void __launch_bounds__(kRecTPB, 1) k_mlp_infer_rec(const float4 *__restrict__ rec, uint32_t n,
+                                                             const uint8_t *__restrict__ img, Params p,
+                                                             __half *__restrict__ probs, int *err) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  SmemInferRec &S = *reinterpret_cast<SmemInferRec *>(smem_raw);
+  const uint32_t g = threadIdx.x >> 7, t = threadIdx.x & 127u, warp = threadIdx.x >> 5;
+  const uint32_t mbar = tc::smem_u32(&S.mbar[g]), mbar_w = tc::smem_u32(&S.mbar_w);
+  if (threadIdx.x == 0) {
+    tc::mbar_init(mbar_w, 1);
+    tc::bulk_load(tc::smem_u32(S.w), img, kImgForward, mbar_w);
+  }
+  if (t == 0) {
+    tc::mbar_init(mbar, 1);
+    S.abort[g] = 0;
+  }
+  if (warp == 0) tc::tmem_alloc(&S.tmem, 512);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = S.tmem + 64u * g, lane_addr = tmem + (((warp & 3u) * 32u) << 16);
+  uint8_t *A = S.a[g];
+  const uint32_t a_addr = tc::smem_u32(A), w_addr = tc::smem_u32(S.w);
+  const uint32_t tries = p.stall_tries ? p.stall_tries : kWaitTries;
+  uint32_t phase = 0;
+  // Few tiles go to different SMs.
+  const uint32_t tile0 = g * gridDim.x + blockIdx.x, stride = gridDim.x * kRecGroups;
+  float4 r0, r1, r2;
+  auto load = [&](uint32_t row) {
+    r0 = r1 = r2 = make_float4(0, 0, 0, 0);
+    if (row >= n) return;
+    r0 = __ldg(rec + 3 * (size_t)row);
+    r1 = __ldg(rec + 3 * (size_t)row + 1);
+    r2 = __ldg(rec + 3 * (size_t)row + 2);
+  };
+  load(tile0 * 128u + t);
+  bool ok = true;
+  for (uint32_t tile = tile0; tile * 128u < n; tile += stride) {
+    const uint32_t row = tile * 128u + t;
+    write_features(A, t, r0, r1, r2, p);
+    load((tile + stride) * 128u + t);
+    if (tile == tile0 && t == 0 && !tc::mbar_wait(mbar_w, 0, kWaitTries)) {
+      S.abort[g] = 1;
+      atomicExch(err, CKR_ERR_ITERATION_LIMIT);
+    }
+    for (int l = 0; l < 4 && ok; ++l) {
+      tc::fence_proxy_async();
+      tc::fence_before_sync();
+      rec_group_sync(g);
+      if (S.abort[g]) {
+        ok = false;  // the weights never arrived
+        break;
+      }
+      if (t == 0 && !(p.stall_tries && l == 0)) {
+        tc::fence_after_sync();
+        if (l == 0) issue(tmem, a_addr, w_addr + kImgW1, kIn, 0);
+        else issue(tmem, a_addr, w_addr + kImgW2 + 10240u * (l - 1), kHidK, 0);
+        tc::mma_commit(mbar);
+      }
+      if (!tc::mbar_wait(mbar, phase, tries)) {
+        S.abort[g] = 1;
+        atomicExch(err, CKR_ERR_ITERATION_LIMIT);
+      }
+      rec_group_sync(g);
+      if (S.abort[g]) {
+        tc::mbar_wait(mbar, phase, tries);  // let the MMAs in flight land before TMEM is freed
+        ok = false;
+        break;
+      }
+      phase ^= 1u;
+      tc::fence_after_sync();
+      if (l < 3) epilogue_relu(lane_addr, A, t);
+    }
+    if (!ok) break;
+    // Softmax over the first C logits, 32 columns at a time: with all 64, exp of the clamped
+    // logit (softmax_exp64), else of its distance from the largest (softmax_exp).
+    const uint32_t C = p.nclusters;
+    float mx = -3.0e38f, sum = 0.f, e[32];
+    if (C != 64)
+      for (int h = 0; h < 2; ++h) {
+        tc::tmem_ld32(lane_addr + 32u * h, e);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+        for (int j = 0; j < 32; ++j)
+          if (32u * h + j < C) mx = fmaxf(mx, e[j]);
+      }
+    auto exps = [&](int h) {
+      tc::tmem_ld32(lane_addr + 32u * h, e);
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        e[j] = C == 64             ? exp_80(fminf(fmaxf(e[j], -80.f), 80.f))
+               : 32u * h + j < C ? __expf(e[j] - mx)
+                                 : 0.f;
+    };
+    for (int h = 0; h < 2; ++h) {
+      exps(h);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) sum += e[j];
+    }
+    const float inv = 1.0f / sum;
+    for (int h = 0; h < 2; ++h) {
+      exps(h);
+      if (row >= n) continue;
+      uint4 *dst = reinterpret_cast<uint4 *>(probs + 64 * (size_t)row + 32 * h);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
         const float *x = e + 8 * q;
         __half2 h0 = __floats2half2_rn(x[0] * inv, x[1] * inv), h1 = __floats2half2_rn(x[2] * inv, x[3] * inv);
         __half2 h2 = __floats2half2_rn(x[4] * inv, x[5] * inv), h3 = __floats2half2_rn(x[6] * inv, x[7] * inv);
@@ -395,13 +538,13 @@ __global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(const float4 *__rest
                             *reinterpret_cast<uint32_t *>(&h2), *reinterpret_cast<uint32_t *>(&h3));
       }
     }
-    if (PATHS) cur = nxt;
     tc::fence_before_sync();
-    group_sync(g);
+    rec_group_sync(g);
   }
+  tc::mbar_wait(mbar_w, 0, kWaitTries);  // a group without a tile: the copy has to land before the block ends
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(S.tmem, 64 * kGroups);
+  if (warp == 0) tc::tmem_dealloc(S.tmem, 512);
 }
 
 // ---- training -------------------------------------------------------------------
@@ -745,8 +888,9 @@ int create(Net &net, uint64_t seed) {
   CKR_CUDA_TRY(cudaMemset(net.err, 0, 4));
   int dev = 0;
   CKR_CUDA_TRY(cudaGetDevice(&dev));
-  for (const void *fn : {(const void *)k_mlp_infer<false>, (const void *)k_mlp_infer<true>}) {
-    CKR_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemInfer)));
+  for (auto [fn, smem] : {std::pair{(const void *)k_mlp_infer, sizeof(SmemInfer)},
+                          std::pair{(const void *)k_mlp_infer_rec, sizeof(SmemInferRec)}}) {
+    CKR_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CKR_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   }
   CKR_CUDA_TRY(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain)));
@@ -776,10 +920,16 @@ int pack(Net &net, cudaStream_t stream) {
   return CKR_OK;
 }
 
-namespace {
-template <bool PATHS>
-int launch_infer(const Net &net, const float4 *rec, const PathRows &pr, uint32_t n_max, const uint32_t *n_dev,
-                 __half *probs, uint16_t *cdf16, float delta, cudaStream_t stream, const uint8_t *img = nullptr) {
+int infer(const Net &net, const float4 *rec, uint32_t n, __half *probs, cudaStream_t stream) {
+  if (n == 0) return CKR_OK;
+  const uint32_t grid = std::min<uint32_t>(ceil_div(n, 128), (uint32_t)sm_count());
+  k_mlp_infer_rec<<<grid, kRecTPB, sizeof(SmemInferRec), stream>>>(rec, n, net.img, params_of(net), probs, net.err);
+  CKR_CUDA_TRY(cudaGetLastError());
+  return CKR_OK;
+}
+
+int infer_paths(const Net &net, const PathRows &rows, uint32_t n_max, const uint32_t *n_dev, uint16_t *cdf16,
+                float delta, cudaStream_t stream, const uint8_t *img) {
   if (n_max == 0) return CKR_OK;
   // CTAs resident per SM: shared memory (the opt-in maximum over the CTA's
   // footprint plus the 1 KB the driver reserves per CTA) or 4.
@@ -790,22 +940,11 @@ int launch_infer(const Net &net, const float4 *rec, const PathRows &pr, uint32_t
     CKR_CUDA_TRY(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     per_sm = std::max(1, std::min(4, smem / (int)(sizeof(SmemInfer) + 1024)));
   }
-  uint32_t grid = std::min<uint32_t>(ceil_div(n_max, 128 * kGroups), (uint32_t)sm_count() * per_sm);
-  k_mlp_infer<PATHS><<<grid, kInferTPB, sizeof(SmemInfer), stream>>>(rec, pr, n_max, n_dev, 0, img ? img : net.img,
-                                                                    params_of(net), delta, probs, cdf16, net.err);
+  const uint32_t grid = std::min<uint32_t>(ceil_div(n_max, 128 * kGroups), (uint32_t)sm_count() * per_sm);
+  k_mlp_infer<<<grid, kInferTPB, sizeof(SmemInfer), stream>>>(rows, n_max, n_dev, img ? img : net.img, params_of(net),
+                                                              delta, cdf16, net.err);
   CKR_CUDA_TRY(cudaGetLastError());
   return CKR_OK;
-}
-}  // namespace
-
-int infer(const Net &net, const float4 *rec, uint32_t n_max, const uint32_t *n_dev, __half *probs, uint16_t *cdf16,
-          float delta, cudaStream_t stream) {
-  return launch_infer<false>(net, rec, PathRows{}, n_max, n_dev, probs, cdf16, delta, stream);
-}
-
-int infer_paths(const Net &net, const PathRows &rows, uint32_t n_max, const uint32_t *n_dev, uint16_t *cdf16,
-                float delta, cudaStream_t stream, const uint8_t *img) {
-  return launch_infer<true>(net, nullptr, rows, n_max, n_dev, nullptr, cdf16, delta, stream, img);
 }
 
 namespace {

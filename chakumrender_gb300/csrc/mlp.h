@@ -57,14 +57,12 @@ struct Net {
 
 int create(Net &net, uint64_t seed);
 void destroy(Net &net);
-// Network output for rows [0, n), n = min(*n_dev, n_max) when n_dev is not null,
-// else n_max; rec: 3 float4 per row.  probs (nullable): the softmax, FP16, 64 per
-// row.  cdf16 (nullable): the selection mixture (1 - delta) softmax + delta / C as
-// 64 cumulative 16-bit entries per row, pmf(j) = (cdf[j] - cdf[j-1]) / 65535.
-int infer(const Net &net, const float4 *rec, uint32_t n_max, const uint32_t *n_dev, __half *probs, uint16_t *cdf16,
-          float delta, cudaStream_t stream);
+// Network output for n records of 3 float4 each: the softmax, FP16, 64 per row.
+int infer(const Net &net, const float4 *rec, uint32_t n, __half *probs, cudaStream_t stream);
 // The selection CDFs for the renderer's queue entries [0, min(*n_dev, n_max)), with
-// the weights of `img` (a copy of Net::img; nullptr: Net::img itself).
+// the weights of `img` (a copy of Net::img; nullptr: Net::img itself): the selection
+// mixture (1 - delta) softmax + delta / C as 64 cumulative 16-bit entries per row, pmf(j) =
+// (cdf[j] - cdf[j-1]) / 65535.
 int infer_paths(const Net &net, const PathRows &rows, uint32_t n_max, const uint32_t *n_dev, uint16_t *cdf16,
                 float delta, cudaStream_t stream, const uint8_t *img = nullptr);
 // One Adam step on the records [0, n) of rec, n = min(*n_dev - n_off, n_max) (rec

@@ -102,8 +102,8 @@ extern "C" int ckr_proposal_infer(ckr_proposal *p, const float *rec12, uint32_t 
   if (!p || (n && (!rec12 || !probs)) || ((uintptr_t)rec12 & 15u) || ((uintptr_t)probs & 15u))
     return CKR_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(p->mu);
-  return mlp::infer(p->net, reinterpret_cast<const float4 *>(rec12), n, nullptr, reinterpret_cast<__half *>(probs),
-                    nullptr, p->defensive, (cudaStream_t)stream);
+  return mlp::infer(p->net, reinterpret_cast<const float4 *>(rec12), n, reinterpret_cast<__half *>(probs),
+                    (cudaStream_t)stream);
 }
 
 extern "C" int ckr_internal_proposal_infer_stalled(ckr_proposal *p, const float *rec12, uint32_t n, uint16_t *probs,
@@ -112,8 +112,8 @@ extern "C" int ckr_internal_proposal_infer_stalled(ckr_proposal *p, const float 
     return CKR_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(p->mu);
   p->net.stall_tries = wait_tries;
-  int st = mlp::infer(p->net, reinterpret_cast<const float4 *>(rec12), n, nullptr, reinterpret_cast<__half *>(probs),
-                      nullptr, p->defensive, (cudaStream_t)stream);
+  int st = mlp::infer(p->net, reinterpret_cast<const float4 *>(rec12), n, reinterpret_cast<__half *>(probs),
+                      (cudaStream_t)stream);
   p->net.stall_tries = 0;
   return st;
 }

@@ -103,9 +103,13 @@ constexpr uint64_t kMbarWaitNs = 1000000000ull;  // 1 s; an MMA chain takes micr
 // Waits for the phase with parity `parity` to complete; gives up after `tries`
 // polls or kMbarWaitNs (returns false) so that a lost arrival cannot hang the GPU.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, uint32_t tries) {
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;  // the clock is read from the 256th poll on: an MMA chain never gets there
   for (uint32_t i = 0; i < tries; ++i) {
-    if ((i & 255u) == 255u && globaltimer_ns() - t0 > kMbarWaitNs) return false;
+    if ((i & 255u) == 255u) {
+      const uint64_t t = globaltimer_ns();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kMbarWaitNs) return false;
+    }
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
