@@ -164,7 +164,7 @@ int enqueue(ckr_batch *b, JobSet &set, bool pack, size_t wave, cudaStream_t stre
   size_t smem = (size_t)depth * TPB * sizeof(uint2);
   // Deep trees: dynamic fetching; one or two levels: one ray per thread.
   const bool dyn = walk_of(s) != kWalkStatic;
-  if (dyn) smem += shear_smem_bytes(TPB);  // the triangle test's ray data
+  if (dyn) smem += dynamic_smem_bytes(TPB);
   const ExtendFn extend_fn = extend_fn_of<TPB>(s);
   const ShadowFn shadow_fn = shadow_fn_of<TPB>(s);
   if (smem > 48 * 1024) {

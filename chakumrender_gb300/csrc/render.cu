@@ -248,7 +248,7 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
   size_t smem = (size_t)depth * kRTPB * sizeof(uint2);
   // Deep trees: dynamic fetching; one or two levels: one ray per thread.
   const bool dyn = walk_of(s) != kWalkStatic;
-  if (dyn) smem += shear_smem_bytes(kRTPB);  // the triangle test's ray data
+  if (dyn) smem += dynamic_smem_bytes(kRTPB);
   const ExtendFn extend_fn = extend_fn_of<kRTPB>(s);
   const ShadowFn shadow_fn = shadow_fn_of<kRTPB>(s);
   if (smem > 48 * 1024) {
@@ -627,7 +627,7 @@ extern "C" int ckr_render_noalloc(ckr_scene *s, const ckr_camera *cam, const ckr
   size_t smem = (size_t)depth * kRTPB * sizeof(uint2);
   // Deep trees: dynamic fetching; one or two levels: one ray per thread.
   const bool dyn = walk_of(s) != kWalkStatic;
-  if (dyn) smem += shear_smem_bytes(kRTPB);  // the triangle test's ray data
+  if (dyn) smem += dynamic_smem_bytes(kRTPB);
   const ExtendFn extend_fn = extend_fn_of<kRTPB>(s);
   const ShadowFn shadow_fn = shadow_fn_of<kRTPB>(s);
   if (smem > 48 * 1024) {

@@ -38,25 +38,15 @@ namespace {
 
 constexpr int kTPB = 128;
 
-// The triangle test's ray data in shared memory after the stacks (TriShearSmem,
-// trace_device.cuh): 64 registers and eight CTAs per SM instead of 72 and seven
-// (closest hit 2.194 -> 2.148 ms per 2^23 rays, any hit 1.621 -> 1.580 ms).  Capping
-// the kernel at 56 or 48 registers (nine or ten CTAs) spilled and was 3 % and 7 %
-// slower.  After them, the 2 KB octant table of the slot bits (slot_lut): the hit
-// bits of each child come from the scene's slot_bits array (2.145 -> 2.105 ms, any
-// hit 1.576 -> 1.546 ms).
-constexpr size_t kAfterStacksBytes = shear_smem_bytes(kTPB) + kSlotLutBytes;
-
 // Closest / any hit over a ray array, with dynamic ray fetching (trace_dynamic).
 template <bool ANY, bool SPHERES, bool DEALT>
-__global__ void __launch_bounds__(kTPB) k_trace_dyn(SceneView s, const float4 *__restrict__ rays, uint32_t n,
+__global__ void __launch_bounds__(kTPB, 8) k_trace_dyn(SceneView s, const float4 *__restrict__ rays, uint32_t n,
                                                     uint32_t *__restrict__ hit_id, float *__restrict__ hit_t,
                                                     uint8_t *__restrict__ occluded, int depth, uint32_t *next,
                                                     uint32_t lanes) {
   extern __shared__ uint2 smem_trav[];
-  float4 *col = shear_column<kTPB>(smem_trav, depth);
-  const uint8_t *lut = fill_slot_lut<kTPB>(reinterpret_cast<uint8_t *>(col - threadIdx.x + 3 * kTPB));
-  const TriShearSmem<kTPB, true, true, SPHERES> tri_pol{col, lut};
+  const auto tri_pol = dynamic_policy<kTPB, SPHERES>(smem_trav, depth);
+  float4 *const col = tri_pol.col;
   auto fetch = [&](uint32_t i, RayPre &r, float &tmax) {
     const float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
     r = make_ray(a, b);
@@ -102,7 +92,7 @@ cudaError_t launch_shape(const ckr_scene *s, LaunchShape &ls) {
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  ls.smem = (size_t)stack_depth_of(s) * kTPB * sizeof(uint2) + kAfterStacksBytes;
+  ls.smem = (size_t)stack_depth_of(s) * kTPB * sizeof(uint2) + dynamic_smem_bytes(kTPB);
   if (ls.smem > 48 * 1024) {
     e = cudaFuncSetAttribute(trace_fn<ANY>(s, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ls.smem);
     if (e != cudaSuccess) return e;

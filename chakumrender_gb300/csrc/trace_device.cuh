@@ -51,16 +51,14 @@ struct RayPre {
 constexpr float kMaxInvDir = 1e20f;
 
 #if defined(__CUDACC__)
-__device__ __forceinline__ float inv_dir(float d) {
-  const float i = 1.0f / d;
-  return fabsf(i) > kMaxInvDir ? copysignf(kMaxInvDir, i) : i;
-}
+__device__ __forceinline__ float cap_inv(float i) { return fabsf(i) > kMaxInvDir ? copysignf(kMaxInvDir, i) : i; }
 
 __device__ __forceinline__ RayPre make_ray(float4 a, float4 b) {
   RayPre r;
   r.ox = a.x; r.oy = a.y; r.oz = a.z; r.tmin = a.w;
   r.dx = b.x; r.dy = b.y; r.dz = b.z;
-  r.ix = inv_dir(r.dx); r.iy = inv_dir(r.dy); r.iz = inv_dir(r.dz);
+  const float i0 = 1.0f / r.dx, i1 = 1.0f / r.dy, i2 = 1.0f / r.dz;
+  r.ix = cap_inv(i0); r.iy = cap_inv(i1); r.iz = cap_inv(i2);
   float ax = fabsf(r.dx), ay = fabsf(r.dy), az = fabsf(r.dz);
   int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
   int kx = kz == 2 ? 0 : kz + 1;
@@ -69,7 +67,7 @@ __device__ __forceinline__ RayPre make_ray(float4 a, float4 b) {
   if (dkz < 0.f) { int t = kx; kx = ky; ky = t; }
   float dkx = kx == 0 ? r.dx : (kx == 1 ? r.dy : r.dz);
   float dky = ky == 0 ? r.dx : (ky == 1 ? r.dy : r.dz);
-  float sx = dkx / dkz, sy = dky / dkz, sz = 1.0f / dkz;
+  float sx = dkx / dkz, sy = dky / dkz, sz = kz == 0 ? i0 : (kz == 1 ? i1 : i2);
   r.mx0 = (kx == 0) ? 1.f : (kz == 0 ? -sx : 0.f);
   r.mx1 = (kx == 1) ? 1.f : (kz == 1 ? -sx : 0.f);
   r.mx2 = (kx == 2) ? 1.f : (kz == 2 ? -sx : 0.f);
@@ -122,20 +120,20 @@ __device__ __forceinline__ bool hit_triangle_sheared(const RayPre &r, const Shea
     W = (float)((double)Bx * (double)Ay - (double)By * (double)Ax);
   }
   if ((U < 0.f || V < 0.f || W < 0.f) && (U > 0.f || V > 0.f || W > 0.f)) return false;
-  float det = U + V + W;
-  if (det == 0.f) return false;
-  float Az = fmaf(m.mz0, a0, fmaf(m.mz1, a1, m.mz2 * a2));
-  float Bz = fmaf(m.mz0, b0, fmaf(m.mz1, b1, m.mz2 * b2));
-  float Cz = fmaf(m.mz0, c0, fmaf(m.mz1, c1, m.mz2 * c2));
-  float T = fmaf(U, Az, fmaf(V, Bz, W * Cz));
-  float t = __fdiv_rn(T, det);
-  if (!(t > r.tmin) || !(t < tbest)) return false;
+  // One branch, on the test that turns most triangles away; the rest decides together.
+  const float det = U + V + W;
+  const float Az = fmaf(m.mz0, a0, fmaf(m.mz1, a1, m.mz2 * a2));
+  const float Bz = fmaf(m.mz0, b0, fmaf(m.mz1, b1, m.mz2 * b2));
+  const float Cz = fmaf(m.mz0, c0, fmaf(m.mz1, c1, m.mz2 * c2));
+  const float T = fmaf(U, Az, fmaf(V, Bz, W * Cz));
+  const float t = __fdiv_rn(T, det);
   // Near-parallel rejection on the unit normal n = (C - A) x (B - A) / |.|.
-  float e10 = v1.x - v0.x, e11 = v1.y - v0.y, e12 = v1.z - v0.z;
-  float e20 = v2.x - v0.x, e21 = v2.y - v0.y, e22 = v2.z - v0.z;
-  float n0 = e21 * e12 - e22 * e11, n1 = e22 * e10 - e20 * e12, n2 = e20 * e11 - e21 * e10;
-  float dn = m.dx * n0 + m.dy * n1 + m.dz * n2;
-  if (dn * dn <= 1e-10f * (n0 * n0 + n1 * n1 + n2 * n2)) return false;
+  const float e10 = v1.x - v0.x, e11 = v1.y - v0.y, e12 = v1.z - v0.z;
+  const float e20 = v2.x - v0.x, e21 = v2.y - v0.y, e22 = v2.z - v0.z;
+  const float n0 = e21 * e12 - e22 * e11, n1 = e22 * e10 - e20 * e12, n2 = e20 * e11 - e21 * e10;
+  const float dn = m.dx * n0 + m.dy * n1 + m.dz * n2;
+  const bool parallel = dn * dn <= 1e-10f * (n0 * n0 + n1 * n1 + n2 * n2);
+  if (det == 0.f || !(t > r.tmin) || !(t < tbest) || parallel) return false;
   t_out = t;
   return true;
 }
@@ -274,7 +272,7 @@ __device__ __forceinline__ void wide_node(const SceneView &s, const RayPre &r, f
     // The plane byte of this slot as the FMA's first operand.
     const uint32_t sel = 0x7604u | ((uint32_t)(slot & 3) << 4);
     auto qf = [&](uint32_t w) {
-      return PERMUTE ? __uint_as_float(__byte_perm(w, 0x3F800000u, sel)) : __uint2float_rn((w >> sh) & 0xffu);
+      return PERMUTE ? __uint_as_float(__byte_perm(w, tri.one, sel)) : __uint2float_rn((w >> sh) & 0xffu);
     };
     const float tnx = __fmaf_rn(qf(nx[h]), sax, nox), tfx = __fmaf_rn(qf(fx[h]), fax, fox);
     const float tny = __fmaf_rn(qf(ny[h]), say, noy), tfy = __fmaf_rn(qf(fy[h]), fay, foy);
@@ -328,11 +326,13 @@ __device__ __forceinline__ Trav trav_start(const SceneView &s, const RayPre &r) 
 // rows and direction (by default the ray's own registers; TriShearSmem reads them
 // from shared memory) and which form of the box test wide_node uses.
 struct TriInRegs {
+  static constexpr bool kInRegs = true;
   static constexpr bool kPermutePlanes = false;
   static constexpr bool kSlotBits = false;
   static constexpr bool kSphereLeaving = true;
   static constexpr bool kSpheres = true;
   const uint8_t *lut = nullptr;
+  uint32_t one = 0x3F800000u;
   __device__ __forceinline__ bool operator()(const RayPre &r, float4 v0, float4 v1, float4 v2, float tbest,
                                              float &t) const {
     return hit_triangle(r, v0, v1, v2, tbest, t);
@@ -344,33 +344,32 @@ __device__ __forceinline__ bool trace_step_rt(const SceneView &s, const RayPre &
                                               Trav &st, uint2 *stack, int stride, int depth, const bool ANY,
                                               Tri tri = Tri{}) {
   // One exit at the end: early returns for the any-hit case split the warp's
-  // control flow and cost more issue slots than the work they skip.
-  bool live = true;
-  if (st.tg.y == 0) {
-    if ((st.ng.y & 0xff000000u) == 0) {
-      if (st.sp == 0)
-        live = false;
-      else
-        st.ng = stack[--st.sp * stride];
-    }
-    if (live) {
-      const uint32_t bit = 31 - __clz(st.ng.y);
-      st.ng.y &= ~(1u << bit);
-      const uint32_t slot = (bit - 24) ^ r.oct;
-      const uint32_t child = st.ng.x + __popc(st.ng.y & ((1u << slot) - 1u) & 0xffu);
-      if (st.ng.y & 0xff000000u) {
-        if (st.sp < depth) {
-          stack[st.sp++ * stride] = st.ng;
-        } else {
-          atomicCAS(s.status, 0, -4 /* CKR_ERR_STACK_OVERFLOW */);
-          best = kMiss;
-          live = false;
-        }
-      }
-      if (live) wide_node<Tri::kPermutePlanes>(s, r, tbest, child, st.ng, st.tg, tri);
+  // control flow and cost more issue slots than the work they skip.  The conditions are
+  // flags, not nested branches, for the same reason (closest hit of 2^23 rays 1.880 ->
+  // 1.837 ms).
+  const bool visit = st.tg.y == 0, pop = visit && (st.ng.y & 0xff000000u) == 0;
+  bool live = !(pop && st.sp == 0);
+  if (pop && live) st.ng = stack[--st.sp * stride];
+  if (visit && live) {
+    const uint32_t bit = 31 - __clz(st.ng.y);
+    st.ng.y &= ~(1u << bit);
+    const uint32_t slot = (bit - 24) ^ r.oct;
+    const uint32_t child = st.ng.x + __popc(st.ng.y & ((1u << slot) - 1u) & 0xffu);
+    const bool push = (st.ng.y & 0xff000000u) != 0;
+    if (push && st.sp >= depth) {
+      atomicCAS(s.status, 0, -4 /* CKR_ERR_STACK_OVERFLOW */);
+      best = kMiss;
+      live = false;
+      st.tg.y = 0;
+    } else {
+      if (push) stack[st.sp++ * stride] = st.ng;
+      wide_node<Tri::kPermutePlanes>(s, r, tbest, child, st.ng, st.tg, tri);
     }
   }
-  if (live && st.tg.y != 0) {
+  // (A finished ray has no triangle pending.  Without the test of `live` the dynamic-fetch
+  // kernels ran at 2.94 ms for 1.84, with it the one-ray-per-thread ones at 753 us for 705
+  // on the box path frame: the compiler joins the warp's lanes elsewhere.)
+  if ((Tri::kInRegs || live) && st.tg.y != 0) {
     const uint32_t k = __ffs(st.tg.y) - 1;
     st.tg.y &= st.tg.y - 1;
     const float4 *tp = s.tris + 3 * (size_t)(st.tg.x + k);
@@ -439,9 +438,10 @@ static __device__ __noinline__ uint32_t trace_ray_rt(const SceneView &s, const R
   return best;
 }
 
-// Lanes of a warp take new work once this many of them are idle (swept: 4 and 16
-// were 4 % and 6 % slower on the 1.3M-triangle workload).
-constexpr int kRefill = 8;
+// Lanes of a warp take new work once this many of them are idle (closest hit of 2^23 rays
+// on 1.3M triangles at 6 / 8 / 10 / 12 / 14 / 16 / 20: 1.867 / 1.833 / 1.825 / 1.819 / 1.829 /
+// 1.901 / 1.962 ms; many-light frame 37.6 / 35.8 / 34.8 / 34.5 / 34.6 / 35.1 / 35.5 ms).
+constexpr int kRefill = 12;
 
 // Few rays: when n rays need no more than the 32 lanes of each of the `warps` resident
 // warps, the launch deals them out itself (trace_dealt), this many to each warp (0: more rays than
@@ -492,6 +492,13 @@ __device__ __forceinline__ void store_shear(float4 *col, const RayPre &r) {
 // by the block at kernel start (the call ends with a block barrier).
 constexpr size_t kSlotLutBytes = 2048;
 
+// A word of shared memory read back, which the compiler cannot take for a literal.
+__device__ __forceinline__ uint32_t opaque_word(volatile uint32_t *smem, uint32_t value) {
+  if (threadIdx.x == 0) *smem = value;
+  __syncthreads();
+  return *smem;
+}
+
 template <int TPB>
 __device__ __forceinline__ const uint8_t *fill_slot_lut(uint8_t *lut) {
   // Bit s to bit s ^ oct: for each bit of oct the halves of its size change places.
@@ -511,14 +518,20 @@ __device__ __forceinline__ const uint8_t *fill_slot_lut(uint8_t *lut) {
 
 // SPHERES: the scene has spheres; without them their code stays out of the refill path
 // (with it, closest hit over 2^23 rays and no sphere took 2.156 ms instead of 2.06).
-template <int TPB, bool PERMUTE, bool SLOTBITS, bool SPHERES>
+template <int TPB, bool SPHERES>
 struct TriShearSmem {
+  static constexpr bool kInRegs = false;
   static constexpr bool kSpheres = SPHERES;
-  static constexpr bool kPermutePlanes = PERMUTE;
-  static constexpr bool kSlotBits = SLOTBITS;
+  static constexpr bool kPermutePlanes = true;
+  static constexpr bool kSlotBits = true;
   static constexpr bool kSphereLeaving = false;
-  const float4 *col;  // this thread's first float4 (shear_column)
+  float4 *col;  // this thread's first float4 (shear_column)
   const uint8_t *lut = nullptr;
+  // The bits of 1.0f, in a register: a literal is set up again for each byte permute (45
+  // moves of the 480 instructions a node visit takes in a warp; closest hit of 2^23 rays
+  // 2.008 -> 1.932 ms).  FFMA2 for the planes, two to an instruction, needs moves and register
+  // ports enough to lose what it saves (2.041 ms with it).
+  uint32_t one = 0x3F800000u;
   __device__ __forceinline__ bool operator()(const RayPre &r, float4 v0, float4 v1, float4 v2, float tbest,
                                              float &t) const {
     const float4 p = col[0], q = col[TPB], u = col[2 * TPB];
@@ -526,6 +539,18 @@ struct TriShearSmem {
     return hit_triangle_sheared(r, m, v0, v1, v2, tbest, t);
   }
 };
+
+// The dynamic-fetch kernels' policy and the shared memory it takes after the stacks: the
+// triangle test's ray data, the octant table, the bits of 1.0f.  All threads must call.
+constexpr size_t dynamic_smem_bytes(int tpb) { return shear_smem_bytes(tpb) + kSlotLutBytes + 16; }
+
+template <int TPB, bool SPHERES>
+__device__ __forceinline__ TriShearSmem<TPB, SPHERES> dynamic_policy(uint2 *smem_stacks, int depth) {
+  float4 *col = shear_column<TPB>(smem_stacks, depth);
+  uint8_t *lut = reinterpret_cast<uint8_t *>(col - threadIdx.x + 3 * TPB);
+  fill_slot_lut<TPB>(lut);
+  return {col, lut, opaque_word(reinterpret_cast<uint32_t *>(lut + kSlotLutBytes), 0x3F800000u)};
+}
 
 template <bool ANY, class Fetch, class Finish, class Tri = TriInRegs>
 __device__ __forceinline__ void trace_dynamic(const SceneView &s, uint32_t n, uint32_t *next, uint2 *stack,
@@ -560,7 +585,7 @@ __device__ __forceinline__ void trace_dynamic(const SceneView &s, uint32_t n, ui
       continue;  // every lane idle: the next iteration refills the whole warp
     }
     if (active) {
-      if (live) live = trace_step<ANY>(s, r, tbest, best, st, stack, stride, depth, tri);
+      if ((!ANY && !Tri::kSpheres) || live) live = trace_step<ANY>(s, r, tbest, best, st, stack, stride, depth, tri);
       if (!live) {
         finish(idx, best, tbest);
         active = false;

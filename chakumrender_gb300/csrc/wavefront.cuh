@@ -298,14 +298,14 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_extend(SceneView s, 
     P.hit_t[slot] = t;
   };
   if constexpr (WALK != kWalkStatic) {
-    float4 *col = shear_column<TPB>(smem_trav, depth);
+    const auto tri = dynamic_policy<TPB, WALK == kWalkDyn>(smem_trav, depth);
     auto fetch_s = [&](uint32_t i, RayPre &r, float &tmax) {
       if (!fetch(i, r, tmax)) return false;
-      store_shear<TPB>(col, r);
+      store_shear<TPB>(tri.col, r);
       return true;
     };
     trace_dynamic<false>(s, P.counts[cur], P.counts + 3, smem_trav + threadIdx.x, TPB, depth, fetch_s, finish,
-                         TriShearSmem<TPB, false, false, WALK == kWalkDyn>{col});
+                         tri);
   } else
     trace_static<false, TPB>(s, P.counts[cur], smem_trav + threadIdx.x, depth, fetch, finish);
 }
@@ -335,14 +335,14 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_shadow(SceneView s, 
     }
   };
   if constexpr (WALK != kWalkStatic) {
-    float4 *col = shear_column<TPB>(smem_trav, depth);
+    const auto tri = dynamic_policy<TPB, WALK == kWalkDyn>(smem_trav, depth);
     auto fetch_s = [&](uint32_t i, RayPre &r, float &tmax) {
       fetch(i, r, tmax);
-      store_shear<TPB>(col, r);
+      store_shear<TPB>(tri.col, r);
       return true;
     };
     trace_dynamic<true>(s, n, P.counts + 4, smem_trav + threadIdx.x, TPB, depth, fetch_s, finish,
-                        TriShearSmem<TPB, false, false, WALK == kWalkDyn>{col});
+                        tri);
   } else
     trace_static<true, TPB>(s, n, smem_trav + threadIdx.x, depth, fetch, finish);
 }
