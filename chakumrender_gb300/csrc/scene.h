@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -97,7 +98,7 @@ struct ckr_scene {
   ckr::DevBuf<uint8_t> st_occ;
   ckr::DevBuf<uint32_t> st_next;  // ray counters of the pipeline streams
   int trace_grid[2] = {1, 1};     // persistent grids of the closest / any-hit kernels
-  cudaMemPool_t counters = nullptr;  // the device's pool of ray counters (trace.cu), shared by its scenes
+  mutable std::atomic<cudaMemPool_t> counters{nullptr};  // pool of the ray counters, once taken (trace.cu)
   size_t trace_smem = 0;          // their traversal stacks
   static constexpr int kMaxPipes = 4;
   cudaStream_t pipe[kMaxPipes] = {};

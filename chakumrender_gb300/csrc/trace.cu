@@ -8,6 +8,7 @@
 // read-only loads.  The host-buffer entry points pipeline uploads, traversal and
 // downloads over internal streams.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstring>
 #include <mutex>
@@ -104,11 +105,11 @@ cudaError_t launch_shape(const ckr_scene *s, LaunchShape &ls) {
   return cudaSuccess;
 }
 
-// The pool the ray counters come from, one per device while that device has scenes.  The
-// device's default pool gives its memory back at every synchronisation, and mapping it
-// again took 180 us of a query that followed one (400,000 rays on 1,280 triangles: 288 us alone, 104 us
-// with this pool and the launches without a counter); this one keeps its single block
-// until the last scene goes.
+// The pool the ray counters come from, one per device while that device has scenes that
+// took counters from it.  The device's default pool gives its memory back at every
+// synchronisation, and mapping it again took 180 us of a query that followed one (400,000
+// rays on 1,280 triangles: 288 us alone, 104 us with this pool); this one keeps its single
+// block until the last of those scenes goes.
 struct CounterPool {
   std::mutex mu;
   cudaMemPool_t pool[64] = {};
@@ -119,12 +120,14 @@ CounterPool &counter_pool() {
   return *p;
 }
 
-// A reference for scene s (released by its destructor's caller); no pool is no error, the
-// counters then come from the default one.
-void counter_pool_add(ckr_scene *s) {
-  if (s->device < 0 || s->device >= 64) return;
+// The pool for scene s, made (100 us) and referenced at the scene's first query that needs a
+// counter; null where there is none, and the counters then come from the default pool.
+cudaMemPool_t counters_of(const ckr_scene *s) {
+  if (cudaMemPool_t p = s->counters.load(std::memory_order_acquire)) return p;
+  if (s->device < 0 || s->device >= 64) return nullptr;
   CounterPool &c = counter_pool();
   std::lock_guard<std::mutex> lock(c.mu);
+  if (cudaMemPool_t p = s->counters.load(std::memory_order_acquire)) return p;
   if (!c.pool[s->device]) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
@@ -134,28 +137,29 @@ void counter_pool_add(ckr_scene *s) {
     uint64_t keep = ~0ull;
     if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
       (void)cudaGetLastError();
-      return;
+      return nullptr;
     }
     if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
       (void)cudaGetLastError();
       cudaMemPoolDestroy(pool);
-      return;
+      return nullptr;
     }
     c.pool[s->device] = pool;
   }
   ++c.refs[s->device];
-  s->counters = c.pool[s->device];
+  s->counters.store(c.pool[s->device], std::memory_order_release);
+  return c.pool[s->device];
 }
 
-void counter_pool_drop(ckr_scene *s) {
-  if (!s->counters) return;
+void counters_drop(ckr_scene *s) {
+  if (!s->counters.load()) return;
   CounterPool &c = counter_pool();
   std::lock_guard<std::mutex> lock(c.mu);
   if (--c.refs[s->device] == 0) {
     cudaMemPoolDestroy(c.pool[s->device]);  // counters still in use keep their memory until freed
     c.pool[s->device] = nullptr;
   }
-  s->counters = nullptr;
+  s->counters.store(nullptr);
 }
 
 // Launches the traversal of rays[0, n).  `next` is a zeroed-per-launch ray counter
@@ -179,10 +183,9 @@ int launch_trace(const ckr_scene *s, const ckr_ray *rays, uint32_t n, uint32_t *
   if (own) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     CKR_CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
-    if (s->counters && capture == cudaStreamCaptureStatusNone)
-      CKR_CUDA_TRY(cudaMallocFromPoolAsync((void **)&next, sizeof(uint32_t), s->counters, stream));
-    else
-      CKR_CUDA_TRY(cudaMallocAsync((void **)&next, sizeof(uint32_t), stream));
+    const cudaMemPool_t pool = capture == cudaStreamCaptureStatusNone ? counters_of(s) : nullptr;
+    if (pool) CKR_CUDA_TRY(cudaMallocFromPoolAsync((void **)&next, sizeof(uint32_t), pool, stream));
+    else CKR_CUDA_TRY(cudaMallocAsync((void **)&next, sizeof(uint32_t), stream));
   }
   cudaError_t e = cudaSuccess;
   constexpr uint32_t kChunk = 1u << 31;
@@ -267,7 +270,6 @@ extern "C" int ckr_scene_create(const float *tri9, uint32_t ntri, const float *s
   if (cudaMemset(s->status.ptr, 0, sizeof(int)) != cudaSuccess) return fail(CKR_ERR_CUDA);
   LaunchShape l0, l1;
   if (launch_shape<false>(s, l0) != cudaSuccess || launch_shape<true>(s, l1) != cudaSuccess) return fail(CKR_ERR_CUDA);
-  counter_pool_add(s);
   s->trace_grid[0] = l0.grid;
   s->trace_grid[1] = l1.grid;
   s->trace_smem = l0.smem;
@@ -286,7 +288,7 @@ extern "C" int ckr_scene_destroy(ckr_scene *scene) {
   if (scene->user_ready) cudaEventDestroy(scene->user_ready);
   if (scene->h_status) cudaFreeHost(scene->h_status);
   if (scene->render_ws && scene->render_ws_free) scene->render_ws_free(scene->render_ws);
-  counter_pool_drop(scene);
+  counters_drop(scene);
   delete scene;
   return CKR_OK;
 }
