@@ -55,6 +55,7 @@ struct ShadeView {
   const float *env_cos;      // env_h + 1: cos(r pi / env_h)
   uint32_t env_w, env_h, env_axis, env_n;
   float env_inv_area;        // 1 / integral of the luminance over the sphere
+  uint32_t finite_radiance;  // every material's radiance and reflectance are finite
 };
 
 }  // namespace ckr
@@ -84,6 +85,7 @@ struct ckr_scene {
   ckr::DevBuf<float> env_marg, env_cond, env_cos;
   uint32_t env_w = 0, env_h = 0, env_axis = 1, env_n = 0;
   float env_inv_area = 0.f;
+  bool finite_radiance = true;
   float bounds[6] = {0, 0, 0, 0, 0, 0};  // scene box (lo.xyz, hi.xyz) of triangles and spheres
   std::vector<ckr_material> host_mats;
   std::vector<ckr::DevLight> host_lights;

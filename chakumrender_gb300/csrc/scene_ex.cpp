@@ -36,6 +36,7 @@ ShadeView shade_view_of(const ckr_scene *s) {
   v.env_axis = s->env_axis;
   v.env_n = s->env_n;
   v.env_inv_area = s->env_inv_area;
+  v.finite_radiance = s->finite_radiance;
   return v;
 }
 
@@ -311,6 +312,9 @@ extern "C" int ckr_scene_create_ex(const ckr_scene_desc *d, ckr_scene **out) {
     s->bounds[3 + c] = lo[c] <= hi[c] ? hi[c] : 0.f;
   }
   s->host_mats.assign(d->materials, d->materials + nm);
+  for (const ckr_material &m : s->host_mats)
+    s->finite_radiance = s->finite_radiance && std::isfinite(m.reflectance) && std::isfinite(m.radiance[0]) &&
+                         std::isfinite(m.radiance[1]) && std::isfinite(m.radiance[2]);
   s->host_lights = lights;
   s->has_shading = true;
   *out = s;

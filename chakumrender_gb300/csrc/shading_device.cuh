@@ -176,12 +176,31 @@ SHD float pdf_eval(const Material &m, F3 n, F3 wo_ref, F3 wo, F3 wi) {
   return s + diffuse;
 }
 
+// A material without a specular part (spec = 0: how these scenes say Lambert) whose GGX term
+// is known to be an exact zero for every direction at least kLambertCos above the surface,
+// seen from wo at cosine co: the term is 0 F D G / (4 cos cos), and with these bounds on
+// roughness, refraction and both cosines F, D and G are finite and the denominators are not
+// zero (the half vector is at least 6e-4 above the surface and at least that much along
+// both directions).  Then brdf = 1 / pi and pdf = cos / pi, bit for bit.
+constexpr float kLambertCos = 2e-4f;
+SHD bool is_lambert(const Material &m, float co) {
+  return m.brdf == kGGX && m.spec == 0.0f && m.alpha >= 1e-2f && m.alpha <= 1e3f && m.ext_ior >= 1e-3f &&
+         m.int_ior >= m.ext_ior && m.int_ior <= 1e5f && co > 1e-3f;
+}
+
 // brdf_eval and pdf_eval of one direction, with the half vector and the distribution
 // (its power or exponential) formed once and one copy of their code: the shading
 // kernels are bound by instruction fetch.  The same operations as the two functions.
-SHD void brdf_pdf_eval(const Material &m, F3 n, F3 wo_ref, F3 wo, F3 wi, float &f, float &p) {
+// `lambert`: is_lambert of the vertex, where most surfaces are (box path frame 704 -> 676 us;
+// the many-light frame, whose mesh is all specular, took 35.5 ms with it and 34.4 without).
+SHD void brdf_pdf_eval(const Material &m, F3 n, F3 wo_ref, F3 wo, F3 wi, float &f, float &p, bool lambert = false) {
   const float diffuse = (1.0f - m.spec) * dot(wi, n) / kPi;
   const float s = m.spec;
+  if (lambert && dot(wi, n) > kLambertCos) {
+    f = 1.0f / kPi;
+    p = diffuse;
+    return;
+  }
   f = 0.0f;
   p = s;
   if (m.brdf == kClassicPhong) {

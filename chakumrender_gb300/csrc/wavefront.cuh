@@ -439,9 +439,10 @@ __device__ __forceinline__ uint32_t may_meet_light(const ShadeView &sv, const Su
 
 // getLightAnalytic / getLightAnalyticDiffuse over every mesh light
 // (src/lightSources_CV.cpp:221-321): spec * amplitude * sum L |I_ltc| / 2pi +
-// (1 - spec) * sum L |I_cos| / 2pi.
+// (1 - spec) * sum L |I_cos| / 2pi.  `no_spec`: the material's spec is 0 and the first part a
+// zero.
 __device__ __forceinline__ F3 ltc_term(const ShadeView &sv, const Surface &S, const Material &M, const LtcLookup &Lk,
-                                       const M3f &minv, bool ltc_on) {
+                                       const M3f &minv, bool ltc_on, bool no_spec = false) {
   F3 G = f3(0, 0, 0);
   for (uint32_t k = 0; k < sv.nlights; ++k) {
     DevLight L = sv.lights[k];
@@ -451,7 +452,7 @@ __device__ __forceinline__ F3 ltc_term(const ShadeView &sv, const Surface &S, co
       const float *t9 = sv.tri9 + 9 * (size_t)(L.first + j);
       F3 A = f3(t9[0], t9[1], t9[2]), B = f3(t9[3], t9[4], t9[5]), C = f3(t9[6], t9[7], t9[8]);
       F3 Le = mat_radiance(sv, sv.tri_mat[L.first + j]);
-      float s = ltc_on ? ltc_spec_tri(A, B, C, S.x, minv) : 0.f;
+      float s = ltc_on && !no_spec ? ltc_spec_tri(A, B, C, S.x, minv) : 0.f;
       float d = ltc_diffuse_tri(A, B, C, S.n, S.x);
       gs = gs + Le * s;
       gd = gd + Le * d;
@@ -544,7 +545,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
     PathCtx pc = path_ctx(prm, 0u);
     uint64_t key = 0;
     F3 o_off = f3(0, 0, 0);
-    bool surface = false;
+    bool surface = false, lam = false;
     if (valid) {
       uint32_t id = P.hit_id[slot];
       meta = P.meta[slot];
@@ -579,6 +580,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
         } else if (!(meta.w & 1u)) {
           surface = true;
           M = material_of(mm);
+          lam = is_lambert(M, dot(S.wo, S.n));
           fcol = f3(mm.color[0], mm.color[1], mm.color[2]) * mm.reflectance;
           key = ckr_key(pc.seed, meta.x - pc.px_base);
           o_off = offset_origin(S.x, S.n);
@@ -645,7 +647,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
               const LightQuery lq = query_lights<true, LF>(sv, S.x, o_off, w, prm.n_light);
               if (last || lq.hit) {
                 float f, p;
-                brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, p);
+                brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, p, lam);
                 if (!last) {
                   const float denom = lq.pdf_sum + (float)nb * p;
                   contrib = mulc(beta, mulc(fcol, lq.Le)) * (f * c / (denom + 1e-20f));
@@ -677,7 +679,12 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
     if (surface && (SHADER == CKR_SHADER_DIRECT_MISCV || SHADER == CKR_SHADER_EXPLICIT)) {
       // getLightFromMeshSource_Analytic_MISCV (src/lightSources_CV.cpp:399-450); at
       // every vertex of the explicit path loop (shadeDI, src/shader.cpp:100-109).
-      F3 G = ltc_term(sv, S, M, Lk, minv, ltc_on);
+      // Without a specular part the BRDF is its LTC approximation (is_lambert: both are 1 / pi),
+      // so a sample's residual is an exact zero and the sample is left out, unless it is a
+      // light's below kLambertCos, which is evaluated to see (a cosine direction never is).
+      // Box, 512^2 x 4 spp: 1.79 -> 0.70 ms.
+      const bool same_brdf = lam && ltc_on && Lk.det > 0.f && Lk.amp < 1e30f && sv.finite_radiance;
+      F3 G = ltc_term(sv, S, M, Lk, minv, ltc_on, same_brdf);
       // MIS residual over the getSamples set; visibility is 1 in the reference.
       F3 res = f3(0, 0, 0);
       const uint32_t nb = prm.n_brdf, nlobe = (uint32_t)((float)nb * M.spec);
@@ -690,7 +697,8 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
         const bool lights = s0 < nls;
         const uint32_t cnt = min(32u, (lights ? nls : nls + nb) - s0);
         uint32_t todo = cnt >= 32 ? 0xffffffffu : (1u << cnt) - 1u;
-        if (!lights) todo = may_meet_light<true>(sv, S, M, key, meta.y, meta.z, o_off, nls, s0 - nls, cnt, nlobe);
+        if (!lights && same_brdf) todo = 0;
+        else if (!lights) todo = may_meet_light<true>(sv, S, M, key, meta.y, meta.z, o_off, nls, s0 - nls, cnt, nlobe);
         while (todo) {
           const uint32_t si = s0 + __ffs(todo) - 1;
           todo &= todo - 1;
@@ -700,12 +708,12 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
           F3 w = lights ? sample_light<LF>(sv, sv.lights[si / prm.n_light], S.x, e0, e1, e2)
                         : sample_dir(M, S.n, S.wo_ref, S.wo, si - nls < nlobe, e1, e2);
           float c = dot(w, S.n);
-          if (c < 0.f) continue;
+          if (c < 0.f || (same_brdf && c > kLambertCos)) continue;
           LightQuery lq = query_lights<false, LF>(sv, S.x, o_off, w, prm.n_light);
           if (lq.mesh == kMiss) continue;
           // lq.mesh: of the first mesh light in list order that the direction meets.
           float f, p;
-          brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, p);
+          brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, w, f, p, lam);
           float denom = lq.pdf_sum + (float)nb * p;
           float fa = f * sv.mats[S.mat].reflectance;
           float fl = ltc_on ? brdf_ltc(M, Lk, minv, S.n, w) * sv.mats[S.mat].reflectance : fa;
