@@ -53,12 +53,17 @@ constexpr float kMaxInvDir = 1e20f;
 #if defined(__CUDACC__)
 __device__ __forceinline__ float cap_inv(float i) { return fabsf(i) > kMaxInvDir ? copysignf(kMaxInvDir, i) : i; }
 
+// BOXES = false: for triangle and sphere tests alone, without the box tests' reciprocals.
+template <bool BOXES = true>
 __device__ __forceinline__ RayPre make_ray(float4 a, float4 b) {
   RayPre r;
   r.ox = a.x; r.oy = a.y; r.oz = a.z; r.tmin = a.w;
   r.dx = b.x; r.dy = b.y; r.dz = b.z;
-  const float i0 = 1.0f / r.dx, i1 = 1.0f / r.dy, i2 = 1.0f / r.dz;
-  r.ix = cap_inv(i0); r.iy = cap_inv(i1); r.iz = cap_inv(i2);
+  float i0 = 0.f, i1 = 0.f, i2 = 0.f;
+  if (BOXES) {
+    i0 = 1.0f / r.dx, i1 = 1.0f / r.dy, i2 = 1.0f / r.dz;
+    r.ix = cap_inv(i0); r.iy = cap_inv(i1); r.iz = cap_inv(i2);
+  }
   float ax = fabsf(r.dx), ay = fabsf(r.dy), az = fabsf(r.dz);
   int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
   int kx = kz == 2 ? 0 : kz + 1;
@@ -67,7 +72,7 @@ __device__ __forceinline__ RayPre make_ray(float4 a, float4 b) {
   if (dkz < 0.f) { int t = kx; kx = ky; ky = t; }
   float dkx = kx == 0 ? r.dx : (kx == 1 ? r.dy : r.dz);
   float dky = ky == 0 ? r.dx : (ky == 1 ? r.dy : r.dz);
-  float sx = dkx / dkz, sy = dky / dkz, sz = kz == 0 ? i0 : (kz == 1 ? i1 : i2);
+  float sx = dkx / dkz, sy = dky / dkz, sz = !BOXES ? 1.0f / dkz : kz == 0 ? i0 : (kz == 1 ? i1 : i2);
   r.mx0 = (kx == 0) ? 1.f : (kz == 0 ? -sx : 0.f);
   r.mx1 = (kx == 1) ? 1.f : (kz == 1 ? -sx : 0.f);
   r.mx2 = (kx == 2) ? 1.f : (kz == 2 ? -sx : 0.f);

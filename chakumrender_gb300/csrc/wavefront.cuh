@@ -497,9 +497,10 @@ __device__ __forceinline__ void cv_samples(const ShadeView &sv, const Paths &P, 
         F3 w = dv * (1.0f / d);
         float c = dot(w, S.n);
         if (!(c < 0.f)) {
-          float c1 = fabsf(dot(w, tri_normal(sv, tri)));
+          const float4 nm = __ldg(&sv.tri_nm[tri]);
+          float c1 = fabsf(dot(w, f3(nm.x, nm.y, nm.z)));
           float g = c * c1 / d2 * w_area;
-          F3 Le = mat_radiance(sv, sv.tri_mat[tri]);
+          F3 Le = mat_radiance(sv, __float_as_uint(nm.w));
           const ckr_material &mm = sv.mats[S.mat];
           float fa = brdf_eval(M, S.n, S.wo_ref, S.wo, w) * mm.reflectance;
           float fl = ltc_on ? brdf_ltc(M, Lk, minv, S.n, w) * mm.reflectance : fa;
@@ -535,8 +536,6 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
     bool valid = i < n;
     uint32_t slot = valid ? q[i] : 0;
     bool cont = false;
-    float4 next_d = make_float4(0, 0, 0, 0), next_b = make_float4(0, 0, 0, 0);
-    F3 next_o = f3(0, 0, 0);
     Surface S;
     Material M;
     F3 fcol = f3(0, 0, 0), beta = f3(0, 0, 0);
@@ -587,6 +586,17 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
         }
       }
     }
+    // The path continues in its slot; its rows are written as soon as they are known: held to
+    // the end of the vertex they were spilled (small-batch pass 1.94 -> 1.87 ms).  A tmin of -1 marks a ray the explicit loop has
+    // traced already.
+    auto go_on = [&](F3 w, F3 nb, float wb) {
+      cont = true;
+      const uint32_t nd = meta.z + 1;
+      P.ray_o[slot] = make_float4(o_off.x, o_off.y, o_off.z, SHADER == CKR_SHADER_EXPLICIT ? -1.f : 0.f);
+      P.ray_d[slot] = make_float4(w.x, w.y, w.z, 3.0e38f);
+      P.beta[slot] = make_float4(nb.x, nb.y, nb.z, wb);
+      P.meta[slot] = make_uint4(meta.x, meta.y, nd, (meta.w & ~1u) | (nd >= pc.max_depth ? 1u : 0u));
+    };
     // ---- direct light ----
     LtcLookup Lk{};
     M3f minv{};
@@ -656,10 +666,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
                 } else if (p > 0.f && f > 0.f) {
                   const float wb = (float)nb * p / ((float)nb * p + lq.pdf_sum);
                   const F3 nbeta = mulc(beta, fcol) * (f * c / (p * (1.0f - prm.rr_prob)));
-                  cont = true;
-                  next_o = o_off;
-                  next_d = make_float4(w.x, w.y, w.z, 3.0e38f);
-                  next_b = make_float4(nbeta.x, nbeta.y, nbeta.z, wb);
+                  go_on(w, nbeta, wb);
                 }
               }
             }
@@ -760,32 +767,21 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
         float f = brdf_eval(M, S.n, S.wo_ref, S.wo, wn) * mm.reflectance;
         float k = 2.0f * kPi * dot(wn, S.n) * f / (1.0f - prm.rr_prob);
         F3 nb = mulc(beta, f3(mm.color[0], mm.color[1], mm.color[2])) * k;
-        cont = true;
-        next_o = o_off;
-        next_d = make_float4(wn.x, wn.y, wn.z, 3.0e38f);
-        next_b = make_float4(nb.x, nb.y, nb.z, 1.f);
+        go_on(wn, nb, 1.f);
         P.hit_id[slot] = hit;
         P.hit_t[slot] = th;
       }
     }
     const bool fresh = regenerate(prm, P, valid && !cont, slot);
     uint32_t cbase = ballot_reserve(&P.counts[cur ^ 1], cont || fresh);
-    if (cont) {
-      // Continue in place: the path keeps its slot.  tmin = -1 marks a ray the
-      // explicit loop has traced already.
-      P.ray_o[slot] = make_float4(next_o.x, next_o.y, next_o.z, SHADER == CKR_SHADER_EXPLICIT ? -1.f : 0.f);
-      P.ray_d[slot] = next_d;
-      P.beta[slot] = next_b;
-      uint32_t nd = meta.z + 1;
-      P.meta[slot] = make_uint4(meta.x, meta.y, nd, (meta.w & ~1u) | (nd >= pc.max_depth ? 1u : 0u));
-    }
     if (cont || fresh) qn[cbase] = slot;
   }
 }
 
-// Shading kernels.  The MIS path tracer's vertex is register hungry but short: at
-// 640 / TPB resident blocks (96 registers at 128 threads, with some spills) the box
-// frame took 1.50 ms against 1.65 ms at the default 149 registers.  The direct-light
+// Shading kernels.  The MIS path tracer's vertex is register hungry but short, and what it
+// spills costs more than resident warps give: at 512 / TPB resident blocks (128 registers at
+// 128 threads, nothing spilled) the box frame takes 628 us, at 640 / 768 / 384 655 / 670 / 684
+// (holding the next ray to the vertex's end, which spilled, 675 at 640).  The direct-light
 // shaders run at 1024 / TPB resident blocks (64 registers at 128 threads): box
 // 512^2 x 4 spp, 10 light + 60 BRDF samples, DIRECT_MIS 10.0 -> 7.8 ms, DIRECT_CV
 // 2.46 -> 2.40 ms against the compiler's choice.  The explicit path loop, which
@@ -805,7 +801,7 @@ __global__ void __launch_bounds__(TPB, shade_blocks(SHADER, TPB)) k_shade(ShadeV
 // LF: the light kinds compiled in (kLightsMeshOnly for scenes whose lights are all
 // MESH / TRI lights, see light_kinds_of).
 template <int TPB, uint32_t LF = kLightsAll>
-__global__ void __launch_bounds__(TPB, (640 / TPB > 1 ? 640 / TPB : 1))
+__global__ void __launch_bounds__(TPB, (512 / TPB > 1 ? 512 / TPB : 1))
     k_shade_path(ShadeView sv0, Paths P, Params prm, int cur, int depth, const LtcEntry *__restrict__ ltc) {
   shade<CKR_SHADER_PATH, TPB, LF>(sv0, P, prm, cur, depth, ltc, SceneView{}, 0);
 }
@@ -819,12 +815,11 @@ inline bool mesh_lights_only(const ckr_scene *s) {
   return true;
 }
 
-// The reference's default shader (MISCV) at 1024 / TPB resident blocks (64
-// registers at 128 threads, with spills): box, 512^2 x 4 spp, 10 light + 60 BRDF
-// samples: 6.13 ms at 512 / TPB (128 registers), 6.24 at 640, 5.89 at 768, 5.51 at
-// 1024, 5.83 at 1280, 5.78 at 1536; at 154 spill-free registers it was slower still.
+// The reference's default shader (MISCV) at 768 / TPB resident blocks (80 registers at
+// 128 threads, with spills): box, 512^2 x 4 spp, 10 light + 60 BRDF samples, at 512 / 640 /
+// 768 / 1024 / 1280: 689 / 684 / 667 / 702 / 752 us.
 template <int TPB, uint32_t LF = kLightsAll>
-__global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
+__global__ void __launch_bounds__(TPB, (768 / TPB > 1 ? 768 / TPB : 1))
     k_shade_miscv(ShadeView sv0, Paths P, Params prm, int cur, int depth, const LtcEntry *__restrict__ ltc) {
   shade<CKR_SHADER_DIRECT_MISCV, TPB, LF>(sv0, P, prm, cur, depth, ltc, SceneView{}, 0);
 }
@@ -835,9 +830,9 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
 // on it; the BRDF sample continues the path and, if it meets an emitter, is
 // weighted at the next vertex with the light technique's pdf of the previous
 // vertex (its pdf is carried in beta.w).  Balance heuristic throughout.  Launched
-// with 1024 / TPB resident blocks (64 registers at 128 threads, some spills): the
-// many-light frame at 640 / 768 / 896 / 1024 was 0.3135 / 0.3110 / 0.3042 /
-// 0.3040 s, the extra resident warps hiding the vertex's dependent loads.
+// with 1024 / TPB resident blocks (64 registers at 128 threads, a few spills): the
+// many-light frame, 1920 x 1080 x 8 spp, at 1024 / 1280 / 1536 takes 34.4 / 35.1 / 36.1 ms,
+// the resident warps hiding the vertex's dependent loads.
 template <int TPB>
 __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
     k_shade_nee(ShadeView sv0, Paths P, Params prm, int cur, Learn lr) {
@@ -855,9 +850,8 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
     const uint32_t slot = valid ? q[i] : 0;
     uint32_t nshadow = 0;
     bool cont = false, rec_ok = false;
-    float4 next_d = make_float4(0, 0, 0, 0), next_b = make_float4(0, 0, 0, 0);
-    float4 so = make_float4(0, 0, 0, 0), sd = so, sc = so, r0 = so, r1 = so, r2 = so;
-    F3 next_o = f3(0, 0, 0);
+    float4 sd = make_float4(0, 0, 0, 0), sc = sd, r0 = sd, r1 = sd, r2 = sd;
+    F3 o_off = f3(0, 0, 0);
     uint4 meta = make_uint4(0, 0, 0, 0);
     ShadeView sv = sv0;  // a batch job's materials replace the scene's
     PathCtx pc = path_ctx(prm, 0u);
@@ -900,7 +894,7 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
           Material M = material_of(mm);
           F3 fcol = f3(mm.color[0], mm.color[1], mm.color[2]) * mm.reflectance;
           uint64_t key = ckr_key(pc.seed, meta.x - pc.px_base);
-          F3 o_off = offset_origin(S.x, S.n);
+          o_off = offset_origin(S.x, S.n);
           // ---- light technique: one sample ----
           float e0 = ckr_draw_f(key, ctr(meta.y, meta.z, 0)), e1 = ckr_draw_f(key, ctr(meta.y, meta.z, 1));
           float e2 = ckr_draw_f(key, ctr(meta.y, meta.z, 2)), e3 = ckr_draw_f(key, ctr(meta.y, meta.z, 3));
@@ -929,7 +923,6 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
               float g = f * c / pl;
               F3 contrib = mulc(beta, mulc(fcol, Le)) * (g * (pl / (pl + pb)));
               nshadow = 1;
-              so = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
               sd = shadow_dir(o_off, Pl);
               sc = make_float4(contrib.x, contrib.y, contrib.z, 0.f);
               if (train_frac > 0.f && ckr_draw_f(key, ctr(meta.y, meta.z, kDimTrain)) < train_frac) {
@@ -956,10 +949,15 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
               brdf_pdf_eval(M, S.n, S.wo_ref, S.wo, wn, f, pb);
               if (pb > 0.f && f > 0.f) {
                 F3 nb = mulc(beta, fcol) * (f * cn / (pb * (1.0f - prm.rr_prob)));
+                // Its rows are written at once: held to the vertex's end they were spilled
+                // (many-light frame 34.4 -> 34.15 ms).
+                const uint32_t nd = meta.z + 1;
                 cont = true;
-                next_o = o_off;
-                next_d = make_float4(wn.x, wn.y, wn.z, 3.0e38f);
-                next_b = make_float4(nb.x, nb.y, nb.z, pb);
+                P.ray_o[slot] = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
+                P.ray_d[slot] = make_float4(wn.x, wn.y, wn.z, 3.0e38f);
+                P.beta[slot] = make_float4(nb.x, nb.y, nb.z, pb);
+                P.meta[slot] = make_uint4(meta.x, meta.y, nd, (meta.w & ~1u) | (nd >= pc.max_depth ? 1u : 0u));
+                if (lr.sel) P.prev_row[slot] = i;
               }
             }
           }
@@ -981,7 +979,7 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
     if (nshadow && sbase >= P.sh_cap) {
       atomicCAS(P.status, 0, CKR_ERR_QUEUE_OVERFLOW);
     } else if (nshadow) {
-      P.sh_o[sbase] = so;
+      P.sh_o[sbase] = make_float4(o_off.x, o_off.y, o_off.z, 0.f);
       P.sh_d[sbase] = sd;
       P.sh_c[sbase] = sc;
       P.sh_px[sbase] = meta.x;
@@ -989,14 +987,6 @@ __global__ void __launch_bounds__(TPB, (1024 / TPB > 1 ? 1024 / TPB : 1))
     }
     const bool fresh = regenerate(prm, P, valid && !cont, slot);
     uint32_t cbase = ballot_reserve(&P.counts[cur ^ 1], cont || fresh);
-    if (cont) {
-      P.ray_o[slot] = make_float4(next_o.x, next_o.y, next_o.z, 0.f);
-      P.ray_d[slot] = next_d;
-      P.beta[slot] = next_b;
-      uint32_t nd = meta.z + 1;
-      P.meta[slot] = make_uint4(meta.x, meta.y, nd, (meta.w & ~1u) | (nd >= pc.max_depth ? 1u : 0u));
-      if (lr.sel) P.prev_row[slot] = i;
-    }
     if (cont || fresh) qn[cbase] = slot;
   }
 }
