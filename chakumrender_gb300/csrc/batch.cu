@@ -98,6 +98,7 @@ struct JobSet {
       J.cam = cam_of(jobs[j].cam);
       J.npix = jobs[j].cam.width * jobs[j].cam.height;
       J.spp = spp_cap ? std::min(jobs[j].spp, spp_cap) : jobs[j].spp;
+      J.inv_spp = 1.0 / J.spp;
       J.max_depth = std::max(1u, jobs[j].max_depth);
       J.mat_off = jobs[j].material_set * nmat;
       J.seed = jobs[j].seed;
