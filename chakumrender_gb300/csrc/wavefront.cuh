@@ -69,9 +69,9 @@ struct Paths {
   uint32_t *prev_row;  // learned selection: the path's row in the previous bounce's probabilities
   uint32_t *sh_rec;    // training: per shadow ray, its training record (kNoRec: none)
   // [0] q[0] length, [1] q[1] length, [2] shadow count, [3] [4] work counters of k_extend
-  // and k_shadow, [5] next camera path to start.  A step's kernels clear them for each
-  // other, in launch order: k_camera and the shading kernel [3], k_extend what the shading
-  // kernel and k_shadow fill (a memset node costs 3 us of a captured step, a memset 1 us).
+  // and k_shadow, [5] next camera path to start, [6] rows that the shading kernel took.  A
+  // step's kernels clear them for each other, in launch order: k_camera and the shading
+  // kernel [3], k_extend what the shading kernel and k_shadow fill (a memset node costs 3 us of a captured step, a memset 1 us).
   uint32_t *counts;
   unsigned long long *stats;  // cumulative closest-hit rays, shadow rays
   double *accum;     // 3 per output pixel
@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(TPB, trace_blocks(TPB)) k_extend(SceneView s, 
     P.counts[cur ^ 1] = 0;
     P.counts[2] = 0;
     P.counts[4] = 0;
+    P.counts[6] = 0;
     atomicAdd(&P.stats[0], (unsigned long long)P.counts[cur]);  // ray statistics: this step's closest-hit rays
   }
   auto fetch = [&](uint32_t i, RayPre &r, float &tmax) {
@@ -522,6 +523,17 @@ __device__ __forceinline__ void cv_samples(const ShadeView &sv, const Paths &P, 
 // of the hemisphere direction at kDimHemi + 2r, + 2r + 1.
 constexpr uint32_t kDimHemi = 1004, kExplicitTries = 8;
 
+// The next 32 queue rows of a warp of a shading kernel, after its first ones: taken from a
+// counter, for a vertex costs from nothing (a miss, an emitter) to all its samples, and warps
+// that strode over the queue ended far apart (512^2 DIRECT_MISCV: 16.9 of 24 warps resident on
+// average, 647 -> 528 us; box path frame 615 -> 606 us; small-batch pass 1822 -> 1798 us).
+__device__ __forceinline__ uint32_t next_rows(const Paths &P, uint32_t stride, uint32_t n, int lane) {
+  if (stride >= n) return n;
+  uint32_t at = 0;
+  if (lane == 0) at = atomicAdd(&P.counts[6], 32u);
+  return stride + __shfl_sync(0xffffffffu, at, 0);
+}
+
 template <uint32_t SHADER, int TPB, uint32_t LF = kLightsAll>
 __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cur, int depth,
                                       const LtcEntry *__restrict__ ltc, SceneView scene, int stack_depth) {
@@ -532,7 +544,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (TPB / 32);
   const uint32_t warp_id = blockIdx.x * (TPB / 32) + (threadIdx.x >> 5);
-  for (uint32_t base = warp_id * 32; base < n; base += warps * 32) {
+  for (uint32_t base = warp_id * 32; base < n; base = next_rows(P, warps * 32, n, lane)) {
     uint32_t i = base + lane;
     bool valid = i < n;
     uint32_t slot = valid ? q[i] : 0;
@@ -817,8 +829,8 @@ inline bool mesh_lights_only(const ckr_scene *s) {
 }
 
 // The reference's default shader (MISCV) at 768 / TPB resident blocks (80 registers at
-// 128 threads, with spills): box, 512^2 x 4 spp, 10 light + 60 BRDF samples, at 512 / 640 /
-// 768 / 1024 / 1280: 689 / 684 / 667 / 702 / 752 us.
+// 128 threads, with spills): box, 512^2 x 4 spp, 10 light + 60 BRDF samples, at 640 / 768 /
+// 1024: 524 / 528 / 535 us.
 template <int TPB, uint32_t LF = kLightsAll>
 __global__ void __launch_bounds__(TPB, (768 / TPB > 1 ? 768 / TPB : 1))
     k_shade_miscv(ShadeView sv0, Paths P, Params prm, int cur, int depth, const LtcEntry *__restrict__ ltc) {
