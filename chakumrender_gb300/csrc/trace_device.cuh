@@ -193,12 +193,12 @@ constexpr float kQuantSlack = 2.384185791015625e-07f;
 // Tests the eight child boxes of wide node `node` (layout in bvh_build.h).  Two
 // forms of the same conservative test: PERMUTE, a plane byte becomes a float
 // through a byte permute folded into the plane's FMA (no integer-to-float
-// conversions on the XU pipe: the traversal kernels, 2.27 -> 2.20 ms per 2^23
+// conversions on the XU pipe: the dynamic-fetch kernels, 2.27 -> 2.20 ms per 2^23
 // rays); otherwise through an integer-to-float conversion, whose per-node set-up
 // needs fewer registers (the renderer's one-ray-per-thread kernels, capped at 64
 // registers, spill with the first form and ran 5-10 % slower).  A slot's hit bits
 // are either assembled from its meta byte or, with Tri::kSlotBits (the traversal
-// kernels), read from the scene's slot_bits array.  Out:
+// kernels with dynamic fetching), read from the scene's slot_bits array.  Out:
 // ng = (child_base, hit interior children at bits 24 + (slot ^ oct) | imask),
 // tg = (tri_base, hit triangles at their offsets from tri_base).
 template <bool PERMUTE, class Tri>
@@ -461,16 +461,6 @@ __host__ __device__ __forceinline__ uint32_t dealt_lanes(uint32_t n, uint32_t wa
   return l < 32u ? l : 32u;
 }
 
-// Traversal loop with dynamic ray fetching (after Aila and Laine, "Understanding
-// the Efficiency of Ray Traversal on GPUs", HPG 2009): a lane whose ray is finished
-// takes the next work item from the global counter `next` (one atomicAdd per warp
-// refill, for as many items as the warp has idle lanes) instead of idling until its
-// whole warp is done; each iteration advances every active lane by one trace_step.
-// Taking 32..128 items per atomic into a warp-private range was 4-5 % slower. The
-// caller zeroes `next` before the launch and runs every lane of every warp through
-// here (the loop votes over full warps).
-//   fetch(i, r, tbest) -> bool: sets up work item i < n (ray, tmax); false skips it.
-//   finish(i, best, tbest): stores the result of item i.
 // The triangle test's ray data (shear rows and direction, Shear) kept in shared
 // memory instead of registers: three float4 per thread in a column of stride TPB
 // after the traversal stacks (depth x TPB uint2), written once per ray by the
@@ -557,6 +547,16 @@ __device__ __forceinline__ TriShearSmem<TPB, SPHERES> dynamic_policy(uint2 *smem
   return {col, lut, opaque_word(reinterpret_cast<uint32_t *>(lut + kSlotLutBytes), 0x3F800000u)};
 }
 
+// Traversal loop with dynamic ray fetching (after Aila and Laine, "Understanding
+// the Efficiency of Ray Traversal on GPUs", HPG 2009): a lane whose ray is finished
+// takes the next work item from the global counter `next` (one atomicAdd per warp
+// refill, for as many items as the warp has idle lanes) instead of idling until its
+// whole warp is done; each iteration advances every active lane by one trace_step.
+// Taking 32..128 items per atomic into a warp-private range was 4-5 % slower. The
+// caller zeroes `next` before the launch and runs every lane of every warp through
+// here (the loop votes over full warps).
+//   fetch(i, r, tbest) -> bool: sets up work item i < n (ray, tmax); false skips it.
+//   finish(i, best, tbest): stores the result of item i.
 template <bool ANY, class Fetch, class Finish, class Tri = TriInRegs>
 __device__ __forceinline__ void trace_dynamic(const SceneView &s, uint32_t n, uint32_t *next, uint2 *stack,
                                               int stride, int depth, Fetch fetch, Finish finish, Tri tri = Tri{}) {

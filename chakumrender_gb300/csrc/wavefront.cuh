@@ -3,8 +3,8 @@
 //
 // Paths occupy path slots.  Each step runs three persistent kernels over
 // device-side queues: k_extend (closest hit), k_shade (emits shadow rays and the
-// continuation ray into queues whose slots are reserved once per warp: a
-// warp-wide prefix sum of the per-lane counts and one atomicAdd by lane 31),
+// continuation ray into queues whose slots are reserved once per warp: a ballot
+// and one atomicAdd by the first lane that wants a slot),
 // k_shadow (any hit, adds unoccluded contributions).  Queue lengths live in device
 // memory.  Paths run in waves (a fixed sequence of launches with no host
 // synchronisation, capturable in a CUDA graph), or, with Params::regen_total set,
@@ -270,7 +270,9 @@ enum Walk : int { kWalkStatic = 0, kWalkDyn = 1, kWalkDynNoSpheres = 2 };
 // rows in registers the kernels took 92 / 89 registers (five CTAs per SM), with them
 // in shared memory 78 / 72 (six / seven CTAs; 1080p 64-spp many-light frame 0.332 ->
 // 0.309 s), and capped at 64 registers without spills, eight CTAs: 0.299 s.  Their
-// box test keeps the conversion form (the permute form at eight CTAs: 0.301 s).
+// box test is the traversal kernels' (plane bytes by permute, the scene's slot bits), the
+// one-ray-per-thread kernels' converts the bytes (with permutes the box frame took 765 us
+// for 701).
 constexpr int trace_blocks(int tpb) { return 1024 / tpb < 1 ? 1 : 1024 / tpb; }
 
 // Closest hit of the paths in queue `cur`.  Dynamic fetching over the queue takes its
