@@ -407,8 +407,10 @@ __device__ __forceinline__ F3 technique_dir(const ShadeView &sv, const Params &p
 // sine, cosine and square root (within 2e-6 of sample_cosine's); the sphere is widened
 // by 2e-4 of its distance and its squared tangent length by 1e-5, well above that and
 // the rounding of these sums.  NaN counts as "may meet".
+// Out of line: the kernels wait on instruction fetch (a 163 x 121 preview 64.2 -> 62.9 us, 512^2
+// DIRECT_MISCV 479 -> 475).
 template <bool MESH_ONLY>
-__device__ __forceinline__ uint32_t may_meet_light(const ShadeView &sv, const Surface &S, const Material &M,
+__device__ __noinline__ uint32_t may_meet_light(const ShadeView &sv, const Surface &S, const Material &M,
                                                    uint64_t key, uint32_t sample, uint32_t depth, F3 o_off,
                                                    uint32_t sidx0, uint32_t i0, uint32_t n, uint32_t nlobe) {
   const uint32_t all = n >= 32 ? 0xffffffffu : (1u << n) - 1u;
@@ -706,6 +708,17 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
       // light's below kLambertCos, which is evaluated to see (a cosine direction never is).
       // Box, 512^2 x 4 spp: 1.79 -> 0.70 ms.
       const bool same_brdf = lam && ltc_on && Lk.det > 0.f && Lk.amp < 1e30f && sv.finite_radiance;
+      // Lights wholly above or below the surface's plane, by more than kLambertCos and the
+      // rounding of a sampled point, have no sample whose cosine must be looked at (521 ->
+      // 477 us).
+      bool no_samples = same_brdf;
+      for (uint32_t k = 0; no_samples && k < sv.first_point; ++k) {
+        const DevLight &L = sv.lights[k];
+        const F3 v = f3(L.px, L.py, L.pz) - S.x;
+        const float r = fabsf(L.radius), h = dot(v, S.n);
+        const float reach = 1e-3f * (length(v) + r) + 1e-6f * (fabsf(L.px) + fabsf(L.py) + fabsf(L.pz) + r);
+        no_samples = h - r > reach || h + r < -reach;
+      }
       F3 G = ltc_term(sv, S, M, Lk, minv, ltc_on, same_brdf);
       // MIS residual over the getSamples set; visibility is 1 in the reference.
       F3 res = f3(0, 0, 0);
@@ -719,7 +732,7 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
         const bool lights = s0 < nls;
         const uint32_t cnt = min(32u, (lights ? nls : nls + nb) - s0);
         uint32_t todo = cnt >= 32 ? 0xffffffffu : (1u << cnt) - 1u;
-        if (!lights && same_brdf) todo = 0;
+        if (lights ? no_samples : same_brdf) todo = 0;
         else if (!lights) todo = may_meet_light<true>(sv, S, M, key, meta.y, meta.z, o_off, nls, s0 - nls, cnt, nlobe);
         while (todo) {
           const uint32_t si = s0 + __ffs(todo) - 1;
