@@ -201,7 +201,9 @@ __global__ void __launch_bounds__(kLtcTPB, 8) k_ltc_shade(const float4 *__restri
     }
   };
   const float inv2pi = 1.0f / (2.0f * kPi);
-  for (uint32_t base = (blockIdx.x * kLtcWarps + warp) * 32u; base < npx; base += gridDim.x * (uint32_t)kLtcTPB) {
+  const uint32_t stride = gridDim.x * (uint32_t)kLtcTPB;
+  for (uint32_t base = (blockIdx.x * kLtcWarps + warp) * 32u; base < npx;
+       base = npx - base > stride ? base + stride : npx) {
     const uint32_t p = base + lane;
     const bool active = p < npx;
     F3 x = f3(0, 0, 0), n = f3(0, 0, 1);
@@ -479,7 +481,12 @@ extern "C" int ckr_ltc_shade(const float *gbuf, uint32_t npx, const float *light
   CKR_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   CKR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLtcTPB, smem));
   if (per_sm < 1) return CKR_ERR_CUDA;
-  int grid = (int)std::min<uint64_t>(ceil_div(npx, kLtcTPB), (uint64_t)sms * per_sm);
+  // Two tiles of pixels to a block once there are more than the resident blocks hold: the
+  // tiles' work differs (how many triangles are clipped), and blocks that stride over 13 tiles
+  // each end far apart.  1024^2 pixels, 8 quads: resident blocks alone 251 us, blocks of four
+  // tiles 245, two 241, one (each staging the emitters) 243.
+  const uint64_t tiles = ceil_div(npx, kLtcTPB);
+  const int grid = (int)std::max(std::min(tiles, (uint64_t)sms * per_sm), tiles / 2);
   fn<<<grid, kLtcTPB, smem, (cudaStream_t)stream>>>(reinterpret_cast<const float4 *>(gbuf), npx, light_tri9, light_rgb,
                                                     nlight, rgb, table);
   CKR_CUDA_TRY(cudaGetLastError());
