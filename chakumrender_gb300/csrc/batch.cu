@@ -172,8 +172,8 @@ int enqueue(ckr_batch *b, JobSet &set, bool pack, size_t wave, cudaStream_t stre
     CKR_CUDA_TRY(cudaFuncSetAttribute(extend_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CKR_CUDA_TRY(cudaFuncSetAttribute(shadow_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
-  const int g_ext = grid_for((const void *)extend_fn, smem, TPB);
-  const int g_sh = grid_for((const void *)shadow_fn, smem, TPB);
+  const int g_ext = walk_grid(walk_of(s), (const void *)extend_fn, smem, TPB);
+  const int g_sh = walk_grid(walk_of(s), (const void *)shadow_fn, smem, TPB);
   const bool nee = b->shader == CKR_SHADER_PATH_NEE;
   void (*const path_fn)(ShadeView, Paths, Params, int, int, const LtcEntry *) =
       mesh_lights_only(s) ? k_shade_path<TPB, kLightsMeshOnly> : k_shade_path<TPB, kLightsAll>;

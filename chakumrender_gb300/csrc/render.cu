@@ -255,8 +255,8 @@ int render_impl(ckr_scene *s, ckr_proposal *prop, const ckr_camera *cam, const c
     CKR_CUDA_TRY(cudaFuncSetAttribute(extend_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CKR_CUDA_TRY(cudaFuncSetAttribute(shadow_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
-  const int g_ext = grid_for((const void *)extend_fn, smem, kRTPB);
-  const int g_sh = grid_for((const void *)shadow_fn, smem, kRTPB);
+  const int g_ext = walk_grid(walk_of(s), (const void *)extend_fn, smem, kRTPB);
+  const int g_sh = walk_grid(walk_of(s), (const void *)shadow_fn, smem, kRTPB);
   const ShadeFn shade = shade_fn_of(s, cfg->shader);
   if (cfg->shader == CKR_SHADER_EXPLICIT && smem > 48 * 1024)
     CKR_CUDA_TRY(cudaFuncSetAttribute(shade.fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -634,8 +634,8 @@ extern "C" int ckr_render_noalloc(ckr_scene *s, const ckr_camera *cam, const ckr
     CKR_CUDA_TRY(cudaFuncSetAttribute(extend_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CKR_CUDA_TRY(cudaFuncSetAttribute(shadow_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
-  const int g_ext = grid_for((const void *)extend_fn, smem, kRTPB);
-  const int g_sh = grid_for((const void *)shadow_fn, smem, kRTPB);
+  const int g_ext = walk_grid(walk_of(s), (const void *)extend_fn, smem, kRTPB);
+  const int g_sh = walk_grid(walk_of(s), (const void *)shadow_fn, smem, kRTPB);
   const ShadeFn shade = shade_fn_of(s, cfg->shader);
   if (cfg->shader == CKR_SHADER_EXPLICIT && smem > 48 * 1024)
     CKR_CUDA_TRY(cudaFuncSetAttribute(shade.fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
