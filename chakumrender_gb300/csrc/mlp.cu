@@ -138,9 +138,10 @@ __device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t *dst, uint
   *reinterpret_cast<uint4 *>(dst + tc::kmaj(t, 72, kHidK)) = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// exp(z) for z in [-80, 80] as 2^(z log2 e): the result is a normal number, so the flushing
-// form of the instruction does, without the scaling around it that __expf needs for
-// denormal results (two multiplies and a compare of every logit).
+// exp(z) for z in [-80, 80] as 2^(z log2 e).  The result is a normal number, so the flushing
+// form of the instruction serves.  Relative error: 2^-22 of the instruction (its PTX
+// specification) and, from the product's rounding, 116 2^-24 ln 2 = 4.8e-6 at |z| = 80;
+// tested through the probabilities, against FP64 (tests/test_proposal.py).
 __device__ __forceinline__ float exp_80(float z) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmul_rn(z, 1.4426950408889634f)));
