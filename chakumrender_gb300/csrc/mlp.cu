@@ -528,15 +528,15 @@ __global__ void __launch_bounds__(kRecTPB, 1) k_mlp_infer_rec(const float4 *__re
     const float inv = 1.0f / sum;
     for (int h = 0; h < 2; ++h) {
       exps(h);
-      if (row >= n) continue;
       uint4 *dst = reinterpret_cast<uint4 *>(probs + 64 * (size_t)row + 32 * h);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const float *x = e + 8 * q;
         __half2 h0 = __floats2half2_rn(x[0] * inv, x[1] * inv), h1 = __floats2half2_rn(x[2] * inv, x[3] * inv);
         __half2 h2 = __floats2half2_rn(x[4] * inv, x[5] * inv), h3 = __floats2half2_rn(x[6] * inv, x[7] * inv);
-        dst[q] = make_uint4(*reinterpret_cast<uint32_t *>(&h0), *reinterpret_cast<uint32_t *>(&h1),
-                            *reinterpret_cast<uint32_t *>(&h2), *reinterpret_cast<uint32_t *>(&h3));
+        const uint4 v = make_uint4(*reinterpret_cast<uint32_t *>(&h0), *reinterpret_cast<uint32_t *>(&h1),
+                                   *reinterpret_cast<uint32_t *>(&h2), *reinterpret_cast<uint32_t *>(&h3));
+        if (row < n) dst[q] = v;
       }
     }
     tc::fence_before_sync();

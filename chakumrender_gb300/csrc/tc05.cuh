@@ -52,14 +52,20 @@ __device__ __forceinline__ uint64_t sdesc_t(uint32_t base, uint32_t C, uint32_t 
   return (uint64_t)((start >> 4) & 0x3FFFu) | (lbo << 16) | (sbo << 32) | (1ull << 46);
 }
 
+// The .sync.aligned instructions below (allocation, loads) want all lanes of the warp at
+// them together, and the code before them branches by lane (a row past the end, the thread
+// that initialises a barrier): each call joins the warp first.
+
 // ---- TMEM allocation (one warp, all lanes) ----
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols) {
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
                "r"(ncols)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
@@ -139,8 +145,9 @@ __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontr
 // Waits until the kernels this launch depends on have ended and their writes are visible.
 __device__ __forceinline__ void wait_dependencies() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// ---- TMEM -> registers: 32 consecutive FP32 columns of this thread's lane ----
+// ---- TMEM -> registers: 32 consecutive FP32 columns of this thread's lane (all lanes) ----
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
+  __syncwarp();
   uint32_t r[32];
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
