@@ -421,7 +421,7 @@ __device__ __noinline__ uint32_t may_meet_light(const ShadeView &sv, const Surfa
     const DevLight &L = sv.lights[k];
     if (MESH_ONLY && L.type != CKR_LIGHT_MESH) continue;
     const F3 l = f3(L.px, L.py, L.pz) - o_off;
-    const float ll = dot(l, l), rr = L.radius + 2e-4f * sqrtf(ll);
+    const float ll = dot(l, l), rr = fabsf(L.radius) + 2e-4f * sqrtf(ll);  // a sphere's radius may be negative
     const float thr = ll - rr * rr - 1e-5f * ll;
     if (!(thr > 0.f)) return all;  // inside or at the sphere
     const float lx = dot(l, X), ly = dot(l, Y), ln = dot(l, S.n);
