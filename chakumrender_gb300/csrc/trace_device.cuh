@@ -344,36 +344,70 @@ struct TriInRegs {
   }
 };
 
+// Takes the group's highest-priority hit child; returns whether any are left.
+__device__ __forceinline__ bool take_child(const RayPre &r, Trav &st, uint32_t &child) {
+  const uint32_t bit = 31 - __clz(st.ng.y);
+  st.ng.y &= ~(1u << bit);
+  const uint32_t slot = (bit - 24) ^ r.oct;
+  child = st.ng.x + __popc(st.ng.y & ((1u << slot) - 1u) & 0xffu);
+  return (st.ng.y & 0xff000000u) != 0;
+}
+
 template <class Tri = TriInRegs>
 __device__ __forceinline__ bool trace_step_rt(const SceneView &s, const RayPre &r, float &tbest, uint32_t &best,
                                               Trav &st, uint2 *stack, int stride, int depth, const bool ANY,
                                               Tri tri = Tri{}) {
   // One exit at the end: early returns for the any-hit case split the warp's
-  // control flow and cost more issue slots than the work they skip.  The conditions are
-  // flags, not nested branches, for the same reason (closest hit of 2^23 rays 1.880 ->
-  // 1.837 ms).
-  const bool visit = st.tg.y == 0, pop = visit && (st.ng.y & 0xff000000u) == 0;
-  bool live = !(pop && st.sp == 0);
-  if (pop && live) st.ng = stack[--st.sp * stride];
-  if (visit && live) {
-    const uint32_t bit = 31 - __clz(st.ng.y);
-    st.ng.y &= ~(1u << bit);
-    const uint32_t slot = (bit - 24) ^ r.oct;
-    const uint32_t child = st.ng.x + __popc(st.ng.y & ((1u << slot) - 1u) & 0xffu);
-    const bool push = (st.ng.y & 0xff000000u) != 0;
-    if (push && st.sp >= depth) {
-      atomicCAS(s.status, 0, -4 /* CKR_ERR_STACK_OVERFLOW */);
-      best = kMiss;
-      live = false;
-      st.tg.y = 0;
-    } else {
-      if (push) stack[st.sp++ * stride] = st.ng;
-      wide_node<Tri::kPermutePlanes>(s, r, tbest, child, st.ng, st.tg, tri);
+  // control flow and cost more issue slots than the work they skip.
+  const bool visit = st.tg.y == 0;
+  bool live = true;
+  if constexpr (Tri::kInRegs) {
+    // One ray per thread: nested branches.  As flags (below) the persistent batch of 128 small
+    // box jobs takes 2.14 ms for 1.27, the box path frame 597 us for 587.
+    if (visit) {
+      if ((st.ng.y & 0xff000000u) == 0) {
+        if (st.sp == 0)
+          live = false;
+        else
+          st.ng = stack[--st.sp * stride];
+      }
+      if (live) {
+        uint32_t child;
+        if (take_child(r, st, child)) {
+          if (st.sp < depth) {
+            stack[st.sp++ * stride] = st.ng;
+          } else {
+            atomicCAS(s.status, 0, -4 /* CKR_ERR_STACK_OVERFLOW */);
+            best = kMiss;
+            live = false;
+          }
+        }
+        if (live) wide_node<Tri::kPermutePlanes>(s, r, tbest, child, st.ng, st.tg, tri);
+      }
+    }
+  } else {
+    // Dynamic fetching: flags (closest hit of 2^23 rays 1.816 ms for 1.859 with the branches
+    // above, many-light frame 34.3 for 35.1).
+    const bool pop = visit && (st.ng.y & 0xff000000u) == 0;
+    live = !(pop && st.sp == 0);
+    if (pop && live) st.ng = stack[--st.sp * stride];
+    if (visit && live) {
+      uint32_t child;
+      const bool push = take_child(r, st, child);
+      if (push && st.sp >= depth) {
+        atomicCAS(s.status, 0, -4 /* CKR_ERR_STACK_OVERFLOW */);
+        best = kMiss;
+        live = false;
+      } else {
+        if (push) stack[st.sp++ * stride] = st.ng;
+        wide_node<Tri::kPermutePlanes>(s, r, tbest, child, st.ng, st.tg, tri);
+      }
     }
   }
-  // (A finished ray has no triangle pending.  Without the test of `live` the dynamic-fetch
-  // kernels ran at 2.94 ms for 1.84, with it the one-ray-per-thread ones at 753 us for 705
-  // on the box path frame: the compiler joins the warp's lanes elsewhere.)
+  // (A ray that finished above has no triangle pending.  Without the test of `live` the
+  // dynamic-fetch kernels ran at 2.94 ms for 1.84, with it the one-ray-per-thread ones take
+  // 593 us for 587 on the box path frame, 1.75 ms for 1.72 on 512 small jobs: the compiler joins
+  // the warp's lanes elsewhere.)
   if ((Tri::kInRegs || live) && st.tg.y != 0) {
     const uint32_t k = __ffs(st.tg.y) - 1;
     st.tg.y &= st.tg.y - 1;
