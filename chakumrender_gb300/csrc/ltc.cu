@@ -6,8 +6,8 @@
 // specular LTC lobe and the diffuse cosine lobe) and its lanes disagree on the
 // path a triangle takes (above, below or across the horizon), so triangles across
 // the horizon are queued per warp and clipped by all lanes together (k_ltc_shade).
-// CTAs are persistent and stride over pixels; the 64x64 LTC table is
-// read from global memory (two entries per pixel), short emitter lists from shared memory.
+// Blocks stride over pixels; the 64x64 LTC table is read from global memory (two entries per
+// pixel), the emitters from shared memory, where each warp stages them 32 at a time (stage_list).
 #include <algorithm>
 
 #include "ckr_internal.h"
@@ -18,18 +18,16 @@
 namespace ckr {
 namespace {
 
-// Blocks of two warps, which share only the emitter list, at 128 registers without spills:
-// 1024^2 pixels and 8 quads take 251 us; four, eight warps a block 250, 254; at ten blocks
-// (96 registers, spills) 258.  Small blocks spread small images: 22 x 771 pixels on 58
+// Blocks of two warps, which share nothing, at 128 registers without spills: 1024^2 pixels and 8
+// quads take 238 us, with four, eight warps a block 239, 252; at ten blocks an SM 235, but 1,000 quads
+// on 5,000 pixels 2.49 ms for 2.39.  Small blocks spread small images: 22 x 771 pixels on 58
 // blocks of eight warps 19.8 us, on 265 blocks of two 10.2.
 constexpr int kLtcTPB = 64, kLtcWarps = kLtcTPB / 32;
 // Deferred triangles per warp and batch of 32 pixels (7.3 KB of shared memory per warp; 384
 // entries at two blocks of 256 threads ran as 256).
 constexpr uint32_t kLtcQueue = 256;
-// Emitter triangles kept in shared memory, 48 bytes each with their radiance: three 16-byte
-// loads a triangle instead of twelve scalar ones (272 -> 266 us, all else alike).  Longer lists
-// are read from global memory.
-constexpr uint32_t kLtcStaged = 64;
+// Distances whose squares may overflow: no test of spheres.
+constexpr float kLtcFar = 1e17f;
 
 // The clipped integrals for a lane whose warp's queue is full.  Out of line: inlined
 // into the classifying loop they pushed it past 128 registers (60 bytes of spills,
@@ -47,12 +45,16 @@ struct GlobalTable {
   SHD LtcEntry operator()(int i) const { return t[i]; }
 };
 
-// Per warp: its 32 pixels' shading frames and the emitter triangles it deferred.
+// Per warp: the emitter triangles at hand (stage_list), its 32 pixels' shading frames and the
+// triangles it deferred.
 struct LtcWarp {
+  float4 tri[32][3];         // (A, r) (B, g) (C, b)
+  float4 group[32];          // a sphere around the group that starts here, its kind in the radius' low bits
   float px[32][17];          // x (3), n (3), Minv in world space (9); padded against bank conflicts
   float res[kLtcQueue][3];   // a deferred triangle's contribution, colour-weighted
   uint2 item[kLtcQueue];     // (lane | light << 5, previous item of the same lane or ~0)
 };
+static_assert(sizeof(LtcWarp) % 16 == 0, "the next warp's rows are 16-byte aligned");
 
 // ---- both lobes at once -------------------------------------------------------------
 // A pair of FP32 numbers in one 64-bit register pair, the specular lobe's in the low half,
@@ -153,6 +155,73 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {
 // Whether two corners of the emitter list are the same point.
 __device__ __forceinline__ bool same(F3 a, F3 b) { return a.x == b.x && a.y == b.y && a.z == b.z; }
 
+// One emitter triangle and its radiance.
+struct LtcTri {
+  F3 A, B, C, col;
+};
+__device__ __forceinline__ LtcTri global_tri(const float *tri9, const float *rgb, uint32_t k) {
+  const float *t = tri9 + 9 * (size_t)k, *c = rgb + 3 * (size_t)k;
+  return {f3(__ldg(t), __ldg(t + 1), __ldg(t + 2)), f3(__ldg(t + 3), __ldg(t + 4), __ldg(t + 5)),
+          f3(__ldg(t + 6), __ldg(t + 7), __ldg(t + 8)), f3(__ldg(c), __ldg(c + 1), __ldg(c + 2))};
+}
+__device__ __forceinline__ LtcTri staged_tri(const LtcWarp &W, uint32_t j) {
+  const float4 a = W.tri[j][0], b = W.tri[j][1], c = W.tri[j][2];
+  return {f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), f3(c.x, c.y, c.z), f3(a.w, b.w, c.w)};
+}
+__device__ __forceinline__ void put_tri(LtcWarp &W, uint32_t j, const LtcTri &t) {
+  W.tri[j][0] = make_float4(t.A.x, t.A.y, t.A.z, t.col.x);
+  W.tri[j][1] = make_float4(t.B.x, t.B.y, t.B.z, t.col.y);
+  W.tri[j][2] = make_float4(t.C.x, t.C.y, t.C.z, t.col.z);
+}
+
+// Kinds of groups: a triangle alone; two that share the edge from their first corner, staged as
+// (a, p, m), (a, m, q); the same, which the list holds in the other order.
+constexpr uint32_t kAlone = 0, kPair = 1, kPairSwapped = 3;
+
+// Stages the triangles [from, from + 32) of the list of n in the warp's shared memory and
+// takes them apart into groups: from the first on, a triangle and the next are a pair if they share
+// the edge.  Returns where the next stage starts: a last triangle with more to come after it may be
+// the first of a pair.  All lanes must call.  Taken apart here, and with pairs in one order, the
+// shading loop has no corners to compare and to choose: 8 quads 245.9 -> 238.1 us (1024^2 pixels), 1,000
+// quads 2.63 -> 2.39 ms (5,000 pixels), one quad 65.7 -> 63.9 us.  16 triangles that share no edge
+// 270 -> 275.
+__device__ __forceinline__ uint32_t stage_list(LtcWarp &W, const float *tri9, const float *rgb, uint32_t from,
+                                               uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u, held = min(32u, n - from);
+  LtcTri t{}, u{};
+  __syncwarp();
+  if (lane < held) put_tri(W, lane, t = global_tri(tri9, rgb, from + lane));
+  __syncwarp();
+  uint32_t kind = kAlone;
+  if (lane + 1 < held) {
+    u = staged_tri(W, lane + 1);
+    if (same(t.A, u.A)) kind = same(t.C, u.B) ? kPair : same(t.B, u.C) ? kPairSwapped : kAlone;
+  }
+  // The second of a pair starts none: the lanes ahead that could start one alternate.
+  const uint32_t could = __ballot_sync(0xffffffffu, kind != kAlone);
+  const uint32_t other = ~could & ((1u << lane) - 1u);  // lanes ahead that could not
+  const bool second = (__clz(other) - (32u - lane)) & 1u;
+  if (second) kind = kAlone;
+  __syncwarp();  // all have read the next one's row
+  if (kind == kPairSwapped) {
+    put_tri(W, lane, u);
+    put_tri(W, lane + 1, t);
+  }
+  // A sphere around the group about its corners' mean; its radius is infinite where a colour is
+  // not finite (whose product with a zero is not zero).
+  const F3 q = kind == kAlone ? t.A : kind == kPair ? u.C : u.B;
+  const F3 c = (t.A + t.B + t.C + q) * 0.25f;
+  auto d2 = [&](F3 p) { return dot(p - c, p - c); };
+  const float rr = max3_nan(max3_nan(d2(t.A), d2(t.B), d2(t.C)), d2(q), 1e-32f);
+  const float r = 1.00001f * rr * rsqrtf(rr);
+  float sum = fabsf(t.col.x) + fabsf(t.col.y) + fabsf(t.col.z);
+  if (kind != kAlone) sum += fabsf(u.col.x) + fabsf(u.col.y) + fabsf(u.col.z);
+  const float w = r < kLtcFar && sum < 3e38f ? r : __int_as_float(0x7f800000);
+  W.group[lane] = make_float4(c.x, c.y, c.z, __uint_as_float((__float_as_uint(w) & ~3u) | kind));
+  __syncwarp();
+  return from + held < n ? from + 31u : n;
+}
+
 // getLightFromMeshSource_Analytic per pixel, one pixel per lane.  Per emitter
 // triangle and lobe a lane settles the triangles wholly above or below its horizon
 // at once; a triangle across the horizon (clipping, four edge integrals) is queued,
@@ -166,10 +235,10 @@ __device__ __forceinline__ bool same(F3 a, F3 b) { return a.x == b.x && a.y == b
 // edge once: 4 corners and 5 edges instead of 6 and 6.  The test is the same for all lanes.
 // Triangles across the horizon are queued by lobe, so that a warp clips one lobe at a time,
 // and clipped without branches (clip_edges); with one mixed queue and a branch per crossed
-// edge the clipping was half of all instructions.  1024^2 pixels, 8 quads: 370 -> 251 us,
-// warp instructions 344 M -> 249 M, active lanes 20.0 -> 26.7 before
-// the emitter list moved to shared memory.
-template <bool STAGED>
+// edge the clipping was half of all instructions.  1024^2 pixels, 8 quads: 370 -> 246 us,
+// warp instructions 344 M -> 249 M, active lanes 20.0 -> 26.7; 238 us with the list taken apart as
+// it is staged (stage_list).
+template <bool FITS>
 __global__ void __launch_bounds__(kLtcTPB, 8) k_ltc_shade(const float4 *__restrict__ gbuf, uint32_t npx,
                                                        const float *__restrict__ light_tri9,
                                                        const float *__restrict__ light_rgb, uint32_t nlight,
@@ -178,28 +247,13 @@ __global__ void __launch_bounds__(kLtcTPB, 8) k_ltc_shade(const float4 *__restri
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   LtcWarp &W = reinterpret_cast<LtcWarp *>(ltc_smem)[warp];
   const GlobalTable tab{table};
-  // Emitter triangle k and its radiance.
-  __shared__ float4 staged[STAGED ? 3 * kLtcStaged : 1];  // (A, r) (B, g) (C, b)
-  if constexpr (STAGED) {
-    for (uint32_t i = threadIdx.x; i < 3 * nlight; i += kLtcTPB)
-      staged[i] = make_float4(light_tri9[3 * i], light_tri9[3 * i + 1], light_tri9[3 * i + 2], light_rgb[i]);
-    __syncthreads();
-  }
-  auto tri = [&](uint32_t k, F3 &A, F3 &B, F3 &C, F3 &col) {
-    if constexpr (STAGED) {
-      const float4 a = staged[3 * k], b = staged[3 * k + 1], c = staged[3 * k + 2];
-      A = f3(a.x, a.y, a.z);
-      B = f3(b.x, b.y, b.z);
-      C = f3(c.x, c.y, c.z);
-      col = f3(a.w, b.w, c.w);
-    } else {
-      const float *t = light_tri9 + 9 * (size_t)k, *c = light_rgb + 3 * (size_t)k;
-      A = f3(__ldg(t), __ldg(t + 1), __ldg(t + 2));
-      B = f3(__ldg(t + 3), __ldg(t + 4), __ldg(t + 5));
-      C = f3(__ldg(t + 6), __ldg(t + 7), __ldg(t + 8));
-      col = f3(__ldg(c), __ldg(c + 1), __ldg(c + 2));
-    }
+  // A list that fits stays staged; its queue items hold staged places, those of a longer one
+  // places in the list.
+  auto fetch = [&](uint32_t k) {
+    if constexpr (FITS) return staged_tri(W, k);
+    else return global_tri(light_tri9, light_rgb, k);
   };
+  uint32_t from = 0, to = 0;  // triangles at hand
   const float inv2pi = 1.0f / (2.0f * kPi);
   const uint32_t stride = gridDim.x * (uint32_t)kLtcTPB;
   for (uint32_t base = (blockIdx.x * kLtcWarps + warp) * 32u; base < npx;
@@ -251,9 +305,8 @@ __global__ void __launch_bounds__(kLtcTPB, 8) k_ltc_shade(const float4 *__restri
             W.item[slot] = make_uint2(lane | k << 5, head);
             head = slot;
           } else {
-            F3 A, B, C, unused;
-            tri(k, A, B, C, unused);
-            const float v = lobe ? clipped_diffuse_here(A, B, C, n, x) : clipped_spec_here(A, B, C, x, minv);
+            const LtcTri t = fetch(k);
+            const float v = lobe ? clipped_diffuse_here(t.A, t.B, t.C, n, x) : clipped_spec_here(t.A, t.B, t.C, x, minv);
             float *acc = lobe ? d3 : s3;
             acc[0] += r * v; acc[1] += g * v; acc[2] += bl * v;
           }
@@ -261,42 +314,46 @@ __global__ void __launch_bounds__(kLtcTPB, 8) k_ltc_shade(const float4 *__restri
         count[lobe] = min(count[lobe] + (uint32_t)__popc(m), kLtcQueue - count[lobe ^ 1u]);
       }
     };
+    // Surfaces that face away from an emitter: a group whose sphere is below both horizons of
+    // every lane adds nothing and is passed over.  Below by a margin several times the rounding of
+    // these sums and of `corner`, so that the corners' own heights come out negative.  A floor of
+    // 1024^2 pixels with 8 quads, all below it 167 -> 60 us, half of them 160 -> 101, all above 160
+    // -> 153 (with a branch per lane ahead of each triangle's edges 118, 154, 201; with a vote on the
+    // corners 101, 131, 168).
+    const F3 z = f3(minv.a[6], minv.a[7], minv.a[8]);
+    const float n2 = dot(n, n), z2 = dot(z, z);
+    float nn = n2 * rsqrtf(n2) * 1.00001f, nz = z2 * rsqrtf(z2) * 1.00001f;
+    if (!active) nn = nz = __int_as_float(0xff800000);  // -inf: below
+    if (!FITS) to = 0;
     for (uint32_t k = 0; k < nlight;) {
-      F3 A, B, C, A2, B2, C2, col, col2;
-      tri(k, A, B, C, col);
-      uint32_t first = k, second = k;  // second == first: no pair
-      F3 pp = B, pm = C, pq = C;
-      if (k + 1 < nlight) {
-        tri(k + 1, A2, B2, C2, col2);
-        if (same(A, A2)) {
-          if (same(C, B2)) {
-            second = k + 1;
-            pq = C2;
-          } else if (same(B, C2)) {
-            first = k + 1;
-            pp = B2;
-            pm = C2;
-            pq = C;
-            const F3 swap = col;
-            col = col2;
-            col2 = swap;
-          }
-        }
+      if (k >= to) {
+        from = k;
+        to = stage_list(W, light_tri9, light_rgb, k, nlight);
       }
-      const Corner a = corner(A, x, n, minv), b = corner(pp, x, n, minv), c = corner(pm, x, n, minv);
+      const uint32_t j = k - from;
+      const float4 g = W.group[j];
+      const uint32_t kind = __float_as_uint(g.w) & 3u;
+      const F3 l = f3(g.x, g.y, g.z) - x;
+      const float l1 = fabsf(l.x) + fabsf(l.y) + fabsf(l.z), m = fmaf(4e-6f, l1, g.w);
+      const float hs = fmaf(z.x, l.x, fmaf(z.y, l.y, fmaf(z.z, l.z, nz * m)));
+      const float hd = fmaf(n.x, l.x, fmaf(n.y, l.y, fmaf(n.z, l.z, nn * m)));
+      const uint32_t k0 = k;
+      k += kind ? 2 : 1;
+      if (__all_sync(0xffffffffu, max3_nan(hs, hd, l1 - kLtcFar) < 0.f)) continue;
+      const uint32_t back = FITS ? 0u : kind >> 1;  // the list's order of a staged pair
+      const LtcTri t = staged_tri(W, j);
+      const Corner a = corner(t.A, x, n, minv), b = corner(t.B, x, n, minv), c = corner(t.C, x, n, minv);
       float s0, d0, s1, d1, sm, dm;
       edge2(a, b, n, s0, d0);
       edge2(b, c, n, s1, d1);
       edge2(c, a, n, sm, dm);
-      add(first, col, a, b, c, s0 + s1 + sm, d0 + d1 + dm);
-      if (first != second) {
-        const Corner q = corner(pq, x, n, minv);
+      add(k0 + back, t.col, a, b, c, s0 + s1 + sm, d0 + d1 + dm);
+      if (kind) {
+        const LtcTri u = staged_tri(W, j + 1);
+        const Corner q = corner(u.C, x, n, minv);
         edge2(c, q, n, s0, d0);
         edge2(q, a, n, s1, d1);
-        add(second, col2, a, c, q, s0 + s1 - sm, d0 + d1 - dm);
-        k += 2;
-      } else {
-        k += 1;
+        add(k0 + 1 - back, u.col, a, c, q, s0 + s1 - sm, d0 + d1 - dm);
       }
     }
     __syncwarp();
@@ -308,20 +365,19 @@ __global__ void __launch_bounds__(kLtcTPB, 8) k_ltc_shade(const float4 *__restri
         const uint2 it = W.item[slot];
         const uint32_t k = it.x >> 5;
         const float *q = W.px[it.x & 31u];
-        F3 A, B, C, col;
-        tri(k, A, B, C, col);
+        const LtcTri t = fetch(k);
         const F3 qx = f3(q[0], q[1], q[2]);
         float v;
         if (lobe) {
-          v = ltc_diffuse_clipped(A, B, C, f3(q[3], q[4], q[5]), qx);
+          v = ltc_diffuse_clipped(t.A, t.B, t.C, f3(q[3], q[4], q[5]), qx);
         } else {
           M3f qm;
           for (int j = 0; j < 9; ++j) qm.a[j] = q[6 + j];
-          v = ltc_spec_clipped(A, B, C, qx, qm);
+          v = ltc_spec_clipped(t.A, t.B, t.C, qx, qm);
         }
-        W.res[slot][0] = col.x * v;
-        W.res[slot][1] = col.y * v;
-        W.res[slot][2] = col.z * v;
+        W.res[slot][0] = t.col.x * v;
+        W.res[slot][1] = t.col.y * v;
+        W.res[slot][2] = t.col.z * v;
       }
     __syncwarp();
     for (uint32_t i = head; i != ~0u; i = W.item[i].y) {
@@ -469,7 +525,7 @@ extern "C" int ckr_ltc_shade(const float *gbuf, uint32_t npx, const float *light
   if (!table) return st;
   if (nlight >= (1u << 26)) return CKR_ERR_TOO_LARGE;  // light index in a queue item
   const size_t smem = kLtcWarps * sizeof(LtcWarp);
-  const auto fn = nlight <= kLtcStaged ? k_ltc_shade<true> : k_ltc_shade<false>;
+  const auto fn = nlight <= 32 ? k_ltc_shade<true> : k_ltc_shade<false>;
   static bool attr_set[64] = {false};
   int dev = 0, sms = 0, per_sm = 0;
   CKR_CUDA_TRY(cudaGetDevice(&dev));
@@ -483,10 +539,11 @@ extern "C" int ckr_ltc_shade(const float *gbuf, uint32_t npx, const float *light
   if (per_sm < 1) return CKR_ERR_CUDA;
   // Two tiles of pixels to a block once there are more than the resident blocks hold: the
   // tiles' work differs (how many triangles are clipped), and blocks that stride over 13 tiles
-  // each end far apart.  1024^2 pixels, 8 quads: resident blocks alone 251 us, blocks of four
-  // tiles 245, two 241, one (each staging the emitters) 243.
+  // each end far apart.  1024^2 pixels, 8 quads: resident blocks alone 241.5 us, blocks of four
+  // tiles 249, two 238, one (each staging the emitters) 240.  Up to eight triangles staging weighs more:
+  // resident blocks alone 63.9 us for 67.7 at one quad, 136.5 for 137.6 at four.
   const uint64_t tiles = ceil_div(npx, kLtcTPB);
-  const int grid = (int)std::max(std::min(tiles, (uint64_t)sms * per_sm), tiles / 2);
+  const int grid = (int)std::max(std::min(tiles, (uint64_t)sms * per_sm), nlight > 8 ? tiles / 2 : 0);
   fn<<<grid, kLtcTPB, smem, (cudaStream_t)stream>>>(reinterpret_cast<const float4 *>(gbuf), npx, light_tri9, light_rgb,
                                                     nlight, rgb, table);
   CKR_CUDA_TRY(cudaGetLastError());
