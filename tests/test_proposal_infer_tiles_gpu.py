@@ -40,7 +40,7 @@ def infer(torch, prop, d_rec, n, calls_of=None):
 
 
 # Rows per SM and group: (tiles per SM, rows more or less).
-@pytest.mark.parametrize("nclusters", [64, 33])
+@pytest.mark.parametrize("nclusters", [64, 33, 8])
 @pytest.mark.parametrize("tiles,more", [(0, 1), (0, 31), (0, 33), (0, 127), (0, 128), (0, 129), (1, 1), (2, -1), (7, -1),
                                         (7, 1), (15, 33)])
 def test_rows_do_not_depend_on_their_tile(torch_cuda, nclusters, tiles, more):
