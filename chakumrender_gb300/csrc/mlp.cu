@@ -148,19 +148,70 @@ __device__ __forceinline__ float exp_ftz(float z) {
   return r;
 }
 
-// exp(z) over the logits of row t when all 64 are clusters, with z clamped to
-// [-80, 80] so that neither the terms nor their sum leave FP32's range (the
-// softmax does not change for logits inside that range); returns the sum.
+// Terms of a softmax over 64 logits without their maximum: exp(z) with z clamped to [-80, 80],
+// so that neither the terms nor their sum leave FP32's range.
+__device__ __forceinline__ float exp_80(float z) { return exp_ftz(fminf(fmaxf(z, -80.f), 80.f)); }
+// Whether the clamp may show in a row whose terms sum to `sum`: a logit of 80 or more
+// (exp(80) = 5.5e34), or none large enough to leave those below -80 (1.8e-35) without weight.
+// Such rows are taken from their maximum instead, exp(z - max), which serves all logits.
+__device__ __forceinline__ bool clamped(float sum) { return !(sum > 1e-20f && sum < 5e34f); }
+// A logit as those rows take it, finite: a NaN as the least.
+__device__ __forceinline__ float finite_logit(float z) { return fminf(fmaxf(z, -3.0e38f), 3.0e38f); }
+
+// exp(z) over the logits of row t when all 64 are clusters; returns the sum.
 __device__ __forceinline__ float softmax_exp64(uint32_t taddr, float *p) {
   tc::tmem_ld32(taddr, p);
   tc::tmem_ld32(taddr + 32, p + 32);
   float sum = 0.f;
 #pragma unroll
   for (int j = 0; j < 64; ++j) {
-    p[j] = exp_ftz(fminf(fmaxf(p[j], -80.f), 80.f));
+    p[j] = exp_80(p[j]);
     sum += p[j];
   }
   return sum;
+}
+
+// Eight probabilities in FP16: terms times `inv`.
+__device__ __forceinline__ uint4 half8(const float *x, float inv) {
+  __half2 h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(x[2 * i] * inv, x[2 * i + 1] * inv);
+  return *reinterpret_cast<uint4 *>(h);
+}
+
+// Cumulative 16-bit table of the selection mixture (1 - delta) softmax + delta / 64: entries
+// j and j + 1 from the terms e, with keep = (1 - delta) / sum and `run` the sum so far.
+__device__ __forceinline__ uint32_t cdf_pair(const float *e, int j, float keep, float unif, float &run) {
+  run += fmaf(keep, e[j], unif);
+  const uint32_t c0 = min(65535u, __float2uint_rn(65535.0f * run));
+  run += fmaf(keep, e[j + 1], unif);
+  const uint32_t c1 = j + 2 == 64 ? 65535u : min(65535u, __float2uint_rn(65535.0f * run));
+  return c0 | (c1 << 16);
+}
+
+// The selection tables of a warp with rows that the clamp would change (`far`): those rows'
+// softmaxes from their maximum, the others' as before; dst null: no row.  Out of line and in local
+// memory, so that it costs the usual warp no registers (frozen learned frame of 640 x 360 x 4
+// 2.07 ms with and without it, 2.08 with it in the kernel).  All lanes must call.
+__device__ __noinline__ void far_cdf(uint32_t taddr, bool far, float delta, uint32_t *dst) {
+  float p[64];
+  tc::tmem_ld32(taddr, p);
+  tc::tmem_ld32(taddr + 32, p + 32);
+  float mx = -3.0e38f, sum = 0.f;
+#pragma unroll 1
+  for (int j = 0; j < 64; ++j) mx = fmaxf(mx, finite_logit(p[j]));
+#pragma unroll 1
+  for (int j = 0; j < 64; ++j) {
+    p[j] = far ? exp_ftz(finite_logit(p[j]) - mx) : exp_80(p[j]);
+    sum += p[j];
+  }
+  const float unif = delta / 64.0f, keep = (1.0f - delta) / sum;
+  float run = 0.f;
+#pragma unroll 1
+  for (int j = 0; j < 64; j += 2) {
+    const uint32_t w = cdf_pair(p, j, keep, unif, run);
+    if (dst) dst[j / 2] = w;
+  }
 }
 
 // exp(z - max) over the first C logits of row t (0 beyond); returns their sum.
@@ -363,18 +414,15 @@ __global__ void __launch_bounds__(kInferTPB, 2) k_mlp_infer(PathRows pr, uint32_
     float e[64];
     const bool full = p.nclusters == 64;
     const float sum = full ? softmax_exp64(lane_addr, e) : softmax_exp(lane_addr, p.nclusters, e);
-    if (row < n && full) {
+    const bool far = full && clamped(sum);
+    if (__any_sync(0xffffffffu, far)) {
+      far_cdf(lane_addr, far, delta, row < n ? reinterpret_cast<uint32_t *>(cdf16 + 64 * (size_t)row) : nullptr);
+    } else if (row < n && full) {
       const float unif = delta / 64.0f, keep = (1.0f - delta) / sum;
       float run = 0.f;
       uint32_t w[32];
 #pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        run += fmaf(keep, e[j], unif);
-        const uint32_t c0 = min(65535u, __float2uint_rn(65535.0f * run));
-        run += fmaf(keep, e[j + 1], unif);
-        const uint32_t c1 = j + 2 == 64 ? 65535u : min(65535u, __float2uint_rn(65535.0f * run));
-        w[j / 2] = c0 | (c1 << 16);
-      }
+      for (int j = 0; j < 64; j += 2) w[j / 2] = cdf_pair(e, j, keep, unif, run);
       uint4 *dst = reinterpret_cast<uint4 *>(cdf16 + 64 * (size_t)row);
 #pragma unroll
       for (int q = 0; q < 8; ++q) dst[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
@@ -502,7 +550,7 @@ __global__ void __launch_bounds__(kRecTPB, 1) k_mlp_infer_rec(const float4 *__re
     }
     if (!ok) break;
     // Softmax over the first C logits, 32 columns at a time: with all 64, exp of the clamped
-    // logit (softmax_exp64), else of its distance from the largest (softmax_exp).  Columns that are
+    // logit (as softmax_exp64), else of its distance from the largest (softmax_exp).  Columns that are
     // no cluster's are not read: 262,144 records with 8 clusters 39.7 -> 32.3 us, with 33
     // 39.6 -> 34.2 (the exp without denormal results).
     const uint32_t C = p.nclusters;
@@ -519,7 +567,7 @@ __global__ void __launch_bounds__(kRecTPB, 1) k_mlp_infer_rec(const float4 *__re
       tc::tmem_ld32(lane_addr + 32u * h, e);
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        e[j] = C == 64           ? exp_ftz(fminf(fmaxf(e[j], -80.f), 80.f))
+        e[j] = C == 64           ? exp_80(e[j])
                : 32u * h + j < C ? exp_ftz(e[j] - mx)
                                  : 0.f;
     };
@@ -528,21 +576,45 @@ __global__ void __launch_bounds__(kRecTPB, 1) k_mlp_infer_rec(const float4 *__re
 #pragma unroll
       for (int j = 0; j < 32; ++j) sum += e[j];
     }
-    const float inv = 1.0f / sum;
-    for (int h = 0; h < 2; ++h) {
-      if (h < halves) exps(h);
-      else
-#pragma unroll
-        for (int j = 0; j < 32; ++j) e[j] = 0.f;
+    const bool far = C == 64 && clamped(sum);
+    auto store = [&](int h, float inv) {
       uint4 *dst = reinterpret_cast<uint4 *>(probs + 64 * (size_t)row + 32 * h);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const float *x = e + 8 * q;
-        __half2 h0 = __floats2half2_rn(x[0] * inv, x[1] * inv), h1 = __floats2half2_rn(x[2] * inv, x[3] * inv);
-        __half2 h2 = __floats2half2_rn(x[4] * inv, x[5] * inv), h3 = __floats2half2_rn(x[6] * inv, x[7] * inv);
-        const uint4 v = make_uint4(*reinterpret_cast<uint32_t *>(&h0), *reinterpret_cast<uint32_t *>(&h1),
-                                   *reinterpret_cast<uint32_t *>(&h2), *reinterpret_cast<uint32_t *>(&h3));
+        const uint4 v = half8(e + 8 * q, inv);
         if (row < n) dst[q] = v;
+      }
+    };
+    if (__any_sync(0xffffffffu, far)) {
+      // As far_cdf, 32 columns at a time in the registers of the usual path (262,144 records 32.8 us
+      // with and without it; out of line, its caller's registers saved, 35.2).
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        tc::tmem_ld32(lane_addr + 32u * h, e);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) mx = fmaxf(mx, finite_logit(e[j]));
+      }
+      sum = 0.f;
+#pragma unroll 1
+      for (int h = 0; h < 4; ++h) {
+        tc::tmem_ld32(lane_addr + 32u * (h & 1), e);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) e[j] = far ? exp_ftz(finite_logit(e[j]) - mx) : exp_80(e[j]);
+        if (h < 2) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum += e[j];
+        } else {
+          store(h - 2, 1.0f / sum);
+        }
+      }
+    } else {
+      const float inv = 1.0f / sum;
+      for (int h = 0; h < 2; ++h) {
+        if (h < halves) exps(h);
+        else
+#pragma unroll
+          for (int j = 0; j < 32; ++j) e[j] = 0.f;
+        store(h, inv);
       }
     }
     tc::fence_before_sync();
