@@ -843,11 +843,11 @@ inline bool mesh_lights_only(const ckr_scene *s) {
   return true;
 }
 
-// The reference's default shader (MISCV) at 768 / TPB resident blocks (80 registers at
-// 128 threads, with spills): box, 512^2 x 4 spp, 10 light + 60 BRDF samples, at 640 / 768 /
-// 1024: 524 / 528 / 535 us.
+// The reference's default shader (MISCV) at 512 / TPB resident blocks (128 registers at
+// 128 threads): box, 512^2 x 4 spp, 10 light + 60 BRDF samples, at 384 / 512 / 640 / 768 / 1024:
+// 487 / 447 / 464 / 469 / 458 us; 200^2 x 3 spp 152 / 160 / 176 / 190 / -.
 template <int TPB, uint32_t LF = kLightsAll>
-__global__ void __launch_bounds__(TPB, (768 / TPB > 1 ? 768 / TPB : 1))
+__global__ void __launch_bounds__(TPB, (512 / TPB > 1 ? 512 / TPB : 1))
     k_shade_miscv(ShadeView sv0, Paths P, Params prm, int cur, int depth, const LtcEntry *__restrict__ ltc) {
   shade<CKR_SHADER_DIRECT_MISCV, TPB, LF>(sv0, P, prm, cur, depth, ltc, SceneView{}, 0);
 }
