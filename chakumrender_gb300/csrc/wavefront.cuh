@@ -254,10 +254,11 @@ __device__ __forceinline__ bool regenerate(const Params &prm, const Paths &P, bo
 }
 
 // Trees at least this many levels deep are traversed with dynamic fetching
-// (trace_dynamic); shallower ones with one ray per thread (trace_static).  Box
-// scene (one level), 256^2 x 16 spp: 1.64 ms static, 1.75 ms dynamic; many-light
-// scene (eight levels), 960x540 x 16 spp: 26.3 ms static, 23.0 ms dynamic.
-constexpr uint32_t kDynamicDepth = 3;
+// (trace_dynamic); shallower ones with one ray per thread (trace_static).  Box scene with more
+// triangles, PATH, 512^2 x 4 spp, static / dynamic: one level (13 triangles) 584 / 760 us, two (21)
+// 761 / 900, three (29) 742 / 895, four (37, 93, 333) 834 / 901, 989 / 978, 1120 / 1050, five
+// (1,293) 1246 / 1118; many-light room, eight levels, 640 x 360 x 4 spp, 1829 / 1546.
+constexpr uint32_t kDynamicDepth = 4;
 
 // How k_extend / k_shadow walk the tree: one ray per thread, or dynamic fetching with
 // or without the scene's spheres.
