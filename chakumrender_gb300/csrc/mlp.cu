@@ -1,15 +1,17 @@
 // mlp.cu — the learned light-selection network on the fifth-generation tensor
-// cores: inference (k_mlp_infer), training forward + backward (k_mlp_train) and
-// the Adam update (k_mlp_adam), all for tiles of 128 rows.
+// cores: inference over the renderer's queue (k_mlp_infer) and on records
+// (k_mlp_infer_rec), training forward + backward (k_mlp_train) and the Adam update
+// (k_mlp_adam), all for tiles of 128 rows.
 //
-// A group of 128 threads owns a tile: thread t computes row t's features and
-// epilogues, thread 0 issues the tcgen05.mma chain of each layer (M = 128 rows,
+// In inference a group of 128 threads owns a tile: thread t computes row t's features and
+// epilogues; in training a block of 256 does, two threads a row.  One thread issues the
+// tcgen05.mma chain of each layer (M = 128 rows,
 // N = 64 outputs, K = 96, or 80 for the hidden layers whose operands carry a
 // constant 1 that multiplies the bias) into tensor memory and commits it to an
 // mbarrier that the group waits on with a bounded poll.  Row t of the
 // accumulator lives in TMEM lane t, which warp (t / 32) % 4 reads with
-// tcgen05.ld.  Inference runs two groups per CTA over the same weights, so one
-// group's epilogue overlaps the other's MMAs; training runs one.
+// tcgen05.ld.  Groups of a CTA share the weights, and one's epilogue overlaps the others'
+// MMAs: two groups over the renderer's queue, seven on records.
 //
 // Backward pass, per layer l with input activations X (rows b) and output
 // gradient G (rows b):  dW^T = X^T G  (M = input features padded to 128,

@@ -4,7 +4,7 @@
 // Paths live in up to `wave` path slots.  Each step runs three persistent kernels
 // over device-side queues: k_extend (closest hit), k_shade (emits shadow rays and
 // the continuation ray into queues whose slots are reserved once per warp: a
-// warp-wide prefix sum of the per-lane counts and one atomicAdd by lane 31),
+// ballot and one atomicAdd by the first lane that wants a slot),
 // k_shadow (any hit, adds unoccluded contributions).  Path tracers of more than
 // one wave regenerate: a path that ends hands its slot to the next camera path,
 // and the host stops on an empty queue.  Otherwise (direct-light shaders, single

@@ -248,10 +248,8 @@ extern "C" int ckr_internal_replay(const float *tri9, uint32_t ntri, uint32_t ma
   return CKR_OK;
 }
 
-// Host-only build with an explicit thread count, for the CPU test suite: an FNV-1a
-// digest of the flattened tree (nodes, then triangle records) and its node count,
-// so that builds on different numbers of threads can be compared.  Not part of the
-// public ABI.
+// The sphere's roots on the host, for the CPU test suite: rows of (o, d, c, r, tmin), mode 0 in
+// pairs of FP32 numbers, 1 in FP64 (sphere_pair.h).  Not part of the public ABI.
 extern "C" int ckr_internal_sphere_roots_host(const float *row, uint32_t n, int mode, float *t, float *rem,
                                               int32_t *code) {
   if (n && (!row || !t || !rem || !code)) return CKR_ERR_INVALID_ARGUMENT;
@@ -273,6 +271,10 @@ extern "C" int ckr_internal_sphere_roots_host(const float *row, uint32_t n, int 
   return CKR_OK;
 }
 
+// Host-only build with an explicit thread count, for the CPU test suite: an FNV-1a
+// digest of the flattened tree (nodes, then triangle records) and its node count,
+// so that builds on different numbers of threads can be compared.  Not part of the
+// public ABI.
 extern "C" int ckr_internal_bvh_digest(const float *tri9, uint32_t ntri, uint32_t max_leaf, uint32_t threads,
                                        uint64_t *digest, uint32_t *nnodes) {
   if (!digest || !nnodes) return CKR_ERR_INVALID_ARGUMENT;

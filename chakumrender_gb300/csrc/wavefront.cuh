@@ -809,13 +809,13 @@ __device__ __forceinline__ void shade(ShadeView sv0, Paths P, Params prm, int cu
 
 // Shading kernels.  The MIS path tracer's vertex is register hungry but short, and what it
 // spills costs more than resident warps give: at 512 / TPB resident blocks (128 registers at
-// 128 threads, nothing spilled) the box frame takes 628 us, at 640 / 768 / 384 655 / 670 / 684
-// (holding the next ray to the vertex's end, which spilled, 675 at 640).  The direct-light
-// shaders run at 1024 / TPB resident blocks (64 registers at 128 threads): box
-// 512^2 x 4 spp, 10 light + 60 BRDF samples, DIRECT_MIS 10.0 -> 7.8 ms, DIRECT_CV
-// 2.46 -> 2.40 ms against the compiler's choice.  The explicit path loop, which
-// traverses inside the kernel, at 512 / TPB (128 registers; box 256^2 x 4 spp,
-// depth 4: 7.01 ms at the compiler's 195 registers, 4.81 ms, 5.06 ms at 640 / TPB).
+// 128 threads, nothing spilled) the box frame takes 586 us, at 640 592 (at 768 / 384, when
+// it took 628, 670 / 684).  The direct-light shaders run at 1024 / TPB resident blocks (64 registers at
+// 128 threads): box, 1080p x 2 spp, DIRECT_MIS of 1 light + 2 BRDF samples, at 512 / 640 / 768 / 1024 /
+// 1280: 835 / 854 / 844 / 821 / 889 us; DIRECT_CV, 17 lights, 256^2, 643 / 635 / 655 / 635 / 668; small
+// frames want fewer (163 x 121 with an environment 58 / 59 / 60 / 63 / 65).  The explicit path loop, which
+// traverses inside the kernel, at 512 / TPB (128 registers; box 192^2 x 4 spp, depth 4, spec
+// 0.6: 301 us, at 384 / 640 328 / 323).
 constexpr int shade_blocks(uint32_t shader, int tpb) {
   return shader == CKR_SHADER_EXPLICIT ? (512 / tpb > 1 ? 512 / tpb : 1) : (1024 / tpb > 1 ? 1024 / tpb : 1);
 }
