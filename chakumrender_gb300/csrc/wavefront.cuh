@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(TPB, shade_blocks(SHADER, TPB)) k_shade(ShadeV
 }
 
 // LF: the light kinds compiled in (kLightsMeshOnly for scenes whose lights are all
-// MESH / TRI lights, see light_kinds_of).
+// MESH / TRI lights, see mesh_lights_only).
 template <int TPB, uint32_t LF = kLightsAll>
 __global__ void __launch_bounds__(TPB, (512 / TPB > 1 ? 512 / TPB : 1))
     k_shade_path(ShadeView sv0, Paths P, Params prm, int cur, int depth, const LtcEntry *__restrict__ ltc) {
